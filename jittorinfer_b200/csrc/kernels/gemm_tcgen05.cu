@@ -1057,6 +1057,54 @@ int auto_splits(long long base_ctas, int num_kb, int bn, int sms) {
     return splits;
 }
 
+// Token-tile width and split count of a plain product of more than 32 tokens: the cheapest pair by a cost model (us) whose constants are
+// a least-squares fit to 315 products x their pairs measured on a B200 (N 160..24576, K 512..16384, 17..2048 tokens, single and gated).
+// What they say: a CTA of one tile costs a start-up that grows with the tile and ~0.2 us per 64 of K (0.36 at 256 tokens), so ONE full
+// wave of small tiles beats half a wave of large ones; two narrow CTAs share an SM at 1.43x; a split costs ~2 us plus its partials;
+// persistent rounds cost less than waves.  Taking the power of two that covers the tokens instead leaves most SMs idle between 33 and
+// ~1000 tokens: 2048 x 2048 at 64 tokens 14.0 -> 7.0 us, at 777 58 -> 13.4 us, 3648 x 2048 at 333 57.9 -> 13.3 us; over all measured
+// shapes that rule is 1.60x the best pair on average, this one 1.02x.
+// Splits of wide tiles need whole SMs of one GPC: past `cap` CTAs the last clusters wait for a second wave (2112 x 5120 at 128 tokens,
+// 64-token tiles: 3 splits = 102 CTAs 16.8 us, 4 splits = 136 CTAs 25.4 us; narrow tiles, two per SM: 272 CTAs fit, 288 do not).
+struct TilePlan {
+    int bn, splits;
+};
+TilePlan plan_tiles(int N, int K, int T, bool dual, bool can_persist, int sms) {
+    static const double start[5] = {2.03, 2.34, 4.48, 6.21, 10.41}, per_kb[5] = {0.194, 0.230, 0.166, 0.210, 0.356};
+    static const double round0[2] = {3.43, 4.62}, round_kb[2] = {0.176, 0.331}, round_end[2] = {2.72, 3.19};
+    const double gate_kb = dual ? 2.7 : 1.0;                      // per 64 of K of a gated pair
+    const int n_tiles = (N + BM - 1) / BM, num_kb = (K + BK - 1) / BK;
+    const double weights = (double) N * K * (dual ? 4 : 2);
+    TilePlan best = {0, 1};
+    double best_us = 1e30;
+    for (int i = 0; i < (dual ? 4 : 5); ++i) {
+        const int bn = 16 << i, occ = bn <= 32 ? 2 : 1;
+        const long long tiles = (long long) n_tiles * ((T + bn - 1) / bn);
+        const double l2_us = 3.0 + (double) tiles * num_kb * (BK * 2) * (BM * (dual ? 2 : 1) + bn) / 18.2e6;
+        const double hbm_us = 3.0 + (weights + 2.0 * T * ((double) K + N)) / 4.26e6;
+        for (int s = 1; s <= 8; ++s) {
+            if (s > 1 && (s > num_kb / 4 || (dual && bn == 32))) break;
+            const int cap = occ == 2 ? sms * (s < 8 ? 184 : 173) / 100 : sms * (s == 3 ? 90 : 82) / 100;
+            if (s > 1 && tiles * s > cap) break;
+            double us;
+            if (s == 1 && bn >= 128 && can_persist && tiles > sms) {
+                const int r = i - 3;
+                us = round0[r] + (double) ((tiles + sms - 1) / sms) * (round_kb[r] * gate_kb * num_kb + round_end[r]);
+            } else {
+                const long long ctas = tiles * s, slots = (long long) sms * occ;
+                const double share = ctas <= sms ? 1.0 : ctas >= slots ? (double) occ : (double) ctas / sms;
+                us = (double) ((ctas + slots - 1) / slots) *
+                     (start[i] + (dual ? 0.3 : 0.0) + per_kb[i] * gate_kb * num_kb / s * (1.0 + 0.434 * (share - 1.0)));
+                if (s > 1) us += 1.82 + 0.053 * bn * (dual ? 2 : 1);
+            }
+            us = us > l2_us ? us : l2_us;
+            us = us > hbm_us ? us : hbm_us;
+            if (us < best_us) { best_us = us; best.bn = bn; best.splits = s; }
+        }
+    }
+    return best;
+}
+
 template <int BN, bool DUAL, int FN>
 int launch_as(const CUtensorMap & a, const CUtensorMap & a2, const CUtensorMap & b, const GemmArgs & args, dim3 grid,
            cudaStream_t stream) {
@@ -1129,7 +1177,22 @@ extern "C" JIB_EXPORT int jib_gemm_bf16(const jib_gemm_desc * d, void * stream_)
     }
     const int n_tiles = (d->N + BM - 1) / BM;
     const int sms = d->sm_count > 0 ? d->sm_count : 148;
-    if (d->bn == 0 && bn == 256 && !grouped && d->ar == nullptr && !d->out_f32 && !jib_no_persist()) {
+    // 16-byte result stores: bf16 rows whose feature offsets keep 16-byte alignment (row pointers of the expert-parallel return
+    // path are row starts of bf16 matrices with d % 8 == 0, hence aligned as well)
+    bool vec_store = !d->out_f32 && d->N % 8 == 0 && d->ldo % 8 == 0 && d->out_batch_stride % 8 == 0 && ((uintptr_t) d->out & 15) == 0 &&
+                     (d->residual == nullptr || (((uintptr_t) d->residual & 15) == 0 && d->ldr % 8 == 0 && d->res_batch_stride % 8 == 0));
+    if (d->ar != nullptr && (((const JibArCtx *) d->ar)->d_max % 8 != 0 || d->out_f32)) vec_store = false;
+    // One matrix, nobody else's choice, more tokens than one narrow tile: the measured cost model chooses.  Up to 32 tokens the split rules
+    // below stand (they are tuned inside decode graphs), and so does the covering tile for matrices of more than two waves of feature tiles
+    // (output heads: every choice streams the weights at the same rate).
+    const bool planned = d->bn == 0 && d->splits <= 0 && !grouped && batch == 1 && d->ar == nullptr && d->ag_flags == nullptr &&
+                         rows_bound > 32 && n_tiles <= 2 * sms;
+    TilePlan plan = {0, 0};
+    if (planned) {
+        plan = plan_tiles(d->N, d->K, rows_bound, dual, vec_store && !jib_no_persist(), sms);
+        bn = plan.bn;
+    }
+    if (!planned && d->bn == 0 && bn == 256 && !grouped && d->ar == nullptr && !d->out_f32 && !jib_no_persist()) {
         // Between one and two waves of 256-token tiles the second wave runs half empty and every CTA pays its prologue and
         // epilogue in the open; the same product as 128-token tiles fills the persistent kernel's two to four rounds evenly
         // with the epilogues hidden (2048 x 2048 x 2048: 25 us -> the persistent form).
@@ -1139,7 +1202,7 @@ extern "C" JIB_EXPORT int jib_gemm_bf16(const jib_gemm_desc * d, void * stream_)
     const int t_tiles = (rows_bound + bn - 1) / bn;
     const int num_kb = (d->K + BK - 1) / BK;
     // split-K: fill the machine when there are too few output tiles
-    int splits = d->splits;
+    int splits = planned ? plan.splits : d->splits;
     const long long base_ctas = (long long) n_tiles * t_tiles * (grouped ? (d->active_hint > 0 ? d->active_hint : batch) : batch);
     if (splits <= 0) splits = d->scratch != nullptr ? auto_splits(base_ctas, num_kb, bn, d->sm_count > 0 ? d->sm_count : 148) : 1;
     // Two ways to add the splits up: inside a thread-block cluster through distributed shared memory (at most 8 CTAs,
@@ -1148,7 +1211,7 @@ extern "C" JIB_EXPORT int jib_gemm_bf16(const jib_gemm_desc * d, void * stream_)
     // tiles x 7 splits (o_proj at TP8) the scratch path is 4.4 us faster.  An explicit split count of up to 8 always
     // takes the cluster (tests exercise both).  Launches with up to 4 splits keep the cluster as well (that is the
     // configuration the single-GPU numbers were measured with).
-    const bool cluster_ok = !jib_no_cluster() && (d->splits > 0 ? d->splits <= 8 : (base_ctas <= 32 || splits <= 4));
+    const bool cluster_ok = !jib_no_cluster() && (planned || (d->splits > 0 ? d->splits <= 8 : (base_ctas <= 32 || splits <= 4)));
     if (d->splits <= 0 && cluster_ok && splits > 8) splits = 8;     // a portable cluster holds at most 8 CTAs
     if (splits > num_kb) splits = num_kb;
     int kbps = (num_kb + splits - 1) / splits;
@@ -1197,12 +1260,7 @@ extern "C" JIB_EXPORT int jib_gemm_bf16(const jib_gemm_desc * d, void * stream_)
     a.expert_list = grouped ? d->expert_list : nullptr;
     a.list_tiles = (grouped && d->expert_list != nullptr && d->list_tiles) ? 1 : 0;
     a.w_evict_first = (t_tiles == 1 && !jib_no_evict_first()) ? 1 : 0;      // one token tile: every weight byte is used once
-    // 16-byte result stores: bf16 rows whose feature offsets keep 16-byte alignment (row pointers of the expert-parallel return
-    // path are row starts of bf16 matrices with d % 8 == 0, hence aligned as well)
-    a.vec_store = (!d->out_f32 && d->N % 8 == 0 && d->ldo % 8 == 0 && d->out_batch_stride % 8 == 0 && ((uintptr_t) d->out & 15) == 0 &&
-                   (d->residual == nullptr || (((uintptr_t) d->residual & 15) == 0 && d->ldr % 8 == 0 && d->res_batch_stride % 8 == 0)))
-                      ? 1 : 0;
-    if (d->ar != nullptr && (((const JibArCtx *) d->ar)->d_max % 8 != 0 || d->out_f32)) a.vec_store = 0;
+    a.vec_store = vec_store ? 1 : 0;
     a.ag_flags = (const unsigned *) d->ag_flags; a.ag_epoch = (const unsigned *) d->ag_epoch;
     a.ag_rows = d->ag_rows; a.ag_world = d->ag_world; a.ar_rs_rows = d->ar_rs_rows;
     a.ag_spin_limit = d->ar != nullptr ? ((const JibArCtx *) d->ar)->spin_limit : 0;
@@ -1229,9 +1287,10 @@ extern "C" JIB_EXPORT int jib_gemm_bf16(const jib_gemm_desc * d, void * stream_)
         if (two_shot && (d->T > ar->max_rows2 || ar->recv2[0] == nullptr || (ar->n_sites & 1) || d->out_f32)) return JIB_E_ARG;
         a.ar = *ar; a.ar_on = two_shot ? 2 : 1; a.ar_site = d->ar_site;
     }
-    // Several waves of wide tiles and nothing but a plain product: the persistent kernel (epilogue under the next tile's MMAs)
+    // More than one wave of wide tiles and nothing but a plain product: the persistent kernel (epilogue under the next tile's MMAs; a second
+    // wave of separate CTAs costs a whole tile more: 3648 x 2048 at 777 tokens, 203 tiles, 25.8 -> 19.8 us)
     if (splits == 1 && a.ar_on == 0 && !src_mode && a.ag_flags == nullptr && a.vec_store && bn >= 128 && !(dual && bn > 128) &&
-        2 * tiles_total >= 3LL * sms && tiles_total < (1LL << 30) && !jib_no_persist()) {
+        tiles_total > sms && tiles_total < (1LL << 30) && !jib_no_persist()) {
         const int n_y = list_tiles ? 1 : t_tiles;
         if (bn == 128) {
             return dual ? launch_persistent<128, true>(ma, ma2, mb, a, n_tiles, n_y, tiles_total, sms, stream)
