@@ -65,6 +65,11 @@ struct FlashArgs {
     float scale_log2e;
 };
 
+__device__ __forceinline__ float warp_max(float v) {
+    asm volatile("redux.sync.max.f32 %0, %0, 0xffffffff;" : "+f"(v));
+    return v;
+}
+
 __device__ __forceinline__ int find_seq(const int * q_start, int n_seqs, int t) {
     int lo = 0, hi = n_seqs;
     while (hi - lo > 1) {
@@ -99,6 +104,7 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     uint64_t * p_ready = s_ready + 1;
     uint64_t * o_ready = p_ready + 1;
     uint32_t * tmem_slot = (uint32_t *) (o_ready + 1);
+    volatile int * failed = (volatile int *) (tmem_slot + 1);    // a softmax warp gave up on a wait: the four leave together
 
     // ---- work description: up to QT distinct sequences among this CTA's tokens ("passes") ----
     // pass j covers the tokens of the group that belong to sequence pass_seq[j]; a column of another sequence is
@@ -166,6 +172,7 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (threadIdx.x == 0) {
         for (int i = 0; i < C::NPAIR; ++i) { mbar_init(&lat_full[i], 1); mbar_init(&lat_free[i], 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(&rope_full[i], 1); mbar_init(&rope_free[i], 1); }
+        *failed = 0;
         mbar_init(q_full, 1);
         mbar_init(s_ready, 1);
         mbar_init(p_ready, 4);
@@ -183,8 +190,20 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     tc_fence_after();
     PDL_TRIGGER_TOP();      // only now: the next grid may start once every CTA of this one holds its tensor-memory columns
     const uint32_t tmem = *tmem_slot;
-    pdl_wait();                                 // q, the latent cache rows written this step, and all outputs
-    JIB_KS(2, 1);
+    if (warp == 0 && elect_one()) {
+        // the first tile's cached rows come out of memory (the weights of a step push them out of L2): asked for ahead of the wait
+        int p = 0;
+        while (pass_k1[p] <= pass_k0[p]) ++p;                       // total_tiles > 0: there is one
+        const int * bt = a.block_tables + (size_t) pass_seq[p] * a.max_blocks;
+        for (int kb = pass_k0[p]; kb < min(pass_k1[p], pass_k0[p] + KV_TILE); kb += BLK) {
+            const int blk = kb / BLK < a.max_blocks ? min(max(bt[kb / BLK], 0), a.n_blocks - 1) : 0;
+#pragma unroll 1
+            for (int c = 0; c < D / 64; ++c) tma_prefetch_2d(&tmKV, c * 64, blk * BLK);
+        }
+    }
+    // q, the latent cache rows written this step, and all outputs: every role waits for them (the softmax warps behind their dry pass)
+    if (warp < 2) pdl_wait();
+    JIB_KS_T(2, 1, 0);
     const uint32_t tm_S = tmem;                 // NQ columns
     const uint32_t tm_O = tmem + NQ;            // 4 x NQ columns
 
@@ -199,7 +218,10 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 const int * bt = a.block_tables + (size_t) pass_seq[p] * a.max_blocks;
                 for (int kb = pass_k0[p]; kb < pass_k1[p] && ok; kb += KV_TILE, ++it) {
                     int blk0 = bt[kb / BLK];
-                    int blk1 = (kb / BLK + 1 < a.max_blocks) ? bt[kb / BLK + 1] : blk0;
+                    // a tile of at most one block of visible rows leaves its second half as it is: those scores are masked and the
+                    // product with the values does not reach them
+                    const int n_blk = pass_k1[p] - kb > BLK ? 2 : 1;
+                    int blk1 = (n_blk == 2 && kb / BLK + 1 < a.max_blocks) ? bt[kb / BLK + 1] : blk0;
                     blk0 = min(max(blk0, 0), a.n_blocks - 1);        // rows past the sequence end are masked later
                     blk1 = min(max(blk1, 0), a.n_blocks - 1);
                     // rope chunk first (the QK product needs all nine chunks, PV only the latent pairs)
@@ -208,9 +230,9 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         const uint32_t ph = (it >> 1) & 1;
                         if (!mbar_wait(&rope_free[s], ph ^ 1)) { jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 21, it); ok = false; break; }
                         uint8_t * dst = rope_ring + s * CHUNK_BYTES;
-                        mbar_expect_tx(&rope_full[s], CHUNK_BYTES);
+                        mbar_expect_tx(&rope_full[s], n_blk * (CHUNK_BYTES / 2));
                         tma_load_2d(dst, &tmKV, &rope_full[s], R, blk0 * BLK);
-                        tma_load_2d(dst + CHUNK_BYTES / 2, &tmKV, &rope_full[s], R, blk1 * BLK);
+                        if (n_blk == 2) tma_load_2d(dst + CHUNK_BYTES / 2, &tmKV, &rope_full[s], R, blk1 * BLK);
                     }
                     for (int m = 0; m < N_LAT_PAIRS && ok; ++m) {
                         const int u = it * N_LAT_PAIRS + m;              // use counter of the pair ring
@@ -218,12 +240,12 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         const uint32_t ph = (u / C::NPAIR) & 1;
                         if (!mbar_wait(&lat_free[s], ph ^ 1)) { jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 22, it); ok = false; break; }
                         uint8_t * dst = ring + s * PAIR_BYTES;
-                        mbar_expect_tx(&lat_full[s], PAIR_BYTES);
+                        mbar_expect_tx(&lat_full[s], n_blk * (PAIR_BYTES / 2));
 #pragma unroll
                         for (int half = 0; half < 2; ++half) {
                             const int x = (2 * m + half) * 64;
                             tma_load_2d(dst + half * CHUNK_BYTES, &tmKV, &lat_full[s], x, blk0 * BLK);
-                            tma_load_2d(dst + half * CHUNK_BYTES + CHUNK_BYTES / 2, &tmKV, &lat_full[s], x, blk1 * BLK);
+                            if (n_blk == 2) tma_load_2d(dst + half * CHUNK_BYTES + CHUNK_BYTES / 2, &tmKV, &lat_full[s], x, blk1 * BLK);
                         }
                     }
                 }
@@ -238,8 +260,12 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             bool ok = mbar_wait(q_full, 0);
             if (!ok) jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 23, 0);
             const uint32_t q_addr = smem_u32(q_s), p_addr = smem_u32(p_s);
-            for (int it = 0; it < total_tiles && ok; ++it) {
+            int p = 0, kb = pass_k0[0];
+            for (int it = 0; it < total_tiles && ok; ++it, kb += KV_TILE) {
+                while (kb >= pass_k1[p]) kb = pass_k0[++p];               // total_tiles counts every pass's tiles: p stays below n_pass
+                const int n_k = min(KV_TILE, pass_k1[p] - kb + 15) / 16;   // 16-row steps with a visible row
                 // ---- S^T = Lat . Q^T over 9 chunks of 64 dims ----
+#pragma unroll 1
                 for (int m = 0; m < N_LAT_PAIRS && ok; ++m) {
                     const int u = it * N_LAT_PAIRS + m;
                     const int s = u % C::NPAIR;
@@ -268,12 +294,12 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 // ---- O^T += Lat^T . P^T ----
                 if (!mbar_wait(p_ready, it & 1)) { jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 26, it); ok = false; break; }
                 tc_fence_after();
+#pragma unroll 1
                 for (int m = 0; m < N_LAT_PAIRS; ++m) {
                     const int u = it * N_LAT_PAIRS + m;
                     const int s = u % C::NPAIR;
                     const uint32_t a_addr = smem_u32(ring + s * PAIR_BYTES);
-#pragma unroll
-                    for (int kk = 0; kk < KV_TILE / 16; ++kk)
+                    for (int kk = 0; kk < n_k; ++kk)
                         mma_bf16(tm_O + m * NQ, desc_mn_sw128(a_addr + kk * 2048, CHUNK_BYTES, 1024),
                                  desc_k_sw128(p_addr + (kk >> 2) * NQ * 128 + (kk & 3) * 32), idesc_pv, (it | kk) != 0);
                     mma_commit(&lat_free[s]);
@@ -291,129 +317,179 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const int row = qd * 32 + lane;               // kv lane (softmax) and output dim inside a 128-dim tile (epilogue)
         const uint32_t lane_addr = (uint32_t) (qd * 32) << 16;
         float m_run[NQ], l_part[NQ];
-#pragma unroll
-        for (int c = 0; c < NQ; ++c) { m_run[c] = -INFINITY; l_part[c] = 0.f; }
         bool ok = true;
-        int it = 0;
-        for (int p = 0; p < n_pass && ok; ++p) {
-            for (int kb = pass_k0[p]; kb < pass_k1[p] && ok; kb += KV_TILE, ++it) {
-                if (!mbar_wait(s_ready, it & 1)) { jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 27, it); ok = false; break; }
+        // A decode CTA runs this code once or twice per launch, and a dozen other kernels between two launches push it out of the
+        // instruction cache: with the first real tile as the first pass, scores to results took 10 us.  So tile -1 is a dry pass over
+        // whatever the buffers hold, while the previous kernel still runs: no waits, no arrivals, no global stores.  For the same reason
+        // the bodies are short (a maximum over a warp is one instruction, 16 columns are added up in 16 exchanges).  From the previous
+        // kernel's end to this one's inside a decode graph, 16 heads: 8 sequences of 1040 rows 11.6 -> 8.0 us; one of up to 64 rows, in
+        // one split, 13.7 and 3.0 us for the merge -> 10.3 us.  What is left is a chain: query and rows in (3 us), two products, results.
+        int it = -1, p = 0, kb = 0;
+        while (true) {
+            const bool dry = it < 0;
+            if (!dry) {
+                if (!mbar_wait(s_ready, it & 1)) { jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 27, it); ok = false; *failed = 1; }
                 tc_fence_after();
                 if (it == 0) JIB_KS_T(2, 4, 64);
-                float s[NQ];
-#pragma unroll
-                for (int c = 0; c < NQ; c += 16) {
-                    uint32_t v[16];
-                    tmem_ld16(tm_S + lane_addr + c, v);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) s[c + j] = __uint_as_float(v[j]);
-                }
-                const int pos = kb + row;
-                // tile max per column over the 128 kv lanes
-#pragma unroll
-                for (int c = 0; c < NQ; ++c) {
-                    const int up = lim[p][c >> 4];
-                    const bool vis = pos < up && (a.window <= 0 || pos >= up - a.window);
-                    float v = vis ? s[c] : -INFINITY;
-                    s[c] = v;
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-                    if (lane == 0) red[qd * NQ + c] = v;
-                }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                float corr[NQ];
-                bool any_corr = false;
-#pragma unroll
-                for (int c = 0; c < NQ; ++c) {
-                    const float mt = fmaxf(fmaxf(red[c], red[NQ + c]), fmaxf(red[2 * NQ + c], red[3 * NQ + c]));
-                    const float m_new = fmaxf(m_run[c], mt);
-                    const float cf = (m_new == -INFINITY) ? 1.f : exp2f((m_run[c] - m_new) * a.scale_log2e);
-                    corr[c] = cf;
-                    any_corr |= cf != 1.f;
-                    const float pv = (s[c] == -INFINITY) ? 0.f : exp2f((s[c] - m_new) * a.scale_log2e);
-                    l_part[c] = l_part[c] * cf + pv;
-                    m_run[c] = m_new;
-                    // P^T[c][row] (bf16) into the swizzled K-major block
-                    const int blk = row >> 6, kcol = row & 63;
-                    const uint32_t off = blk * (NQ * 128) + c * 128 + ((((kcol * 2) >> 4) ^ (c & 7)) << 4) + ((kcol * 2) & 15);
-                    *(bf16 *) (p_s + off) = __float2bfloat16(pv);
-                }
-                // running-max correction of O^T (previous PV products must have landed)
-                if (it > 0) {
-                    if (!mbar_wait(o_ready, (it - 1) & 1)) { jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 28, it); ok = false; }
-                    tc_fence_after();
-                    if (any_corr && ok) {
-#pragma unroll 1
-                        for (int m = 0; m < N_LAT_PAIRS; ++m)
-#pragma unroll
-                            for (int c = 0; c < NQ; c += 16) {
-                                uint32_t v[16];
-                                tmem_ld16(tm_O + lane_addr + m * NQ + c, v);
-                                tmem_ld_wait();
-#pragma unroll
-                                for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * corr[c + j]);
-                                tmem_st16(tm_O + lane_addr + m * NQ + c, v);
-                            }
-                        tmem_st_wait();
-                    }
-                }
-                fence_proxy_async();          // P^T stores -> visible to the tensor core's async-proxy reads
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(p_ready);
-                asm volatile("bar.sync 1, 128;" ::: "memory");   // red[] reuse in the next tile
             }
-        }
-        // ---- epilogue ----
-        if (ok && !mbar_wait(o_ready, (total_tiles - 1) & 1)) { jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 29, 0); ok = false; }
-        tc_fence_after();
-        // l per column = sum over the 128 kv lanes
-        float l_tot[NQ];
+            if (it <= 0) {
 #pragma unroll
-        for (int c = 0; c < NQ; ++c) {
-            float v = l_part[c];
+                for (int c = 0; c < NQ; ++c) { m_run[c] = -INFINITY; l_part[c] = 0.f; }
+            }
+            float s[NQ];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) red[qd * NQ + c] = v;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+            for (int c = 0; c < NQ; c += 16) {
+                uint32_t v[16];
+                tmem_ld16(tm_S + lane_addr + c, v);
+                tmem_ld_wait();
 #pragma unroll
-        for (int c = 0; c < NQ; ++c) l_tot[c] = red[c] + red[NQ + c] + red[2 * NQ + c] + red[3 * NQ + c];
-        if (ok) {
+                for (int j = 0; j < 16; ++j) s[c + j] = __uint_as_float(v[j]);
+            }
+            const int pos = kb + row;
+            // tile max per column over the 128 kv lanes; lane c keeps column c's maximum of this warp
+            float keep = -INFINITY;
+#pragma unroll
+            for (int c = 0; c < NQ; ++c) {
+                const int up = lim[p][c >> 4];
+                const bool vis = pos < up && (a.window <= 0 || pos >= up - a.window);
+                s[c] = vis ? s[c] : -INFINITY;
+                const float v = warp_max(s[c]);
+                if (lane == c) keep = v;
+            }
+            if (lane < NQ) red[lane * 4 + qd] = keep;
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            float corr[NQ];
+            bool any_corr = false;
+#pragma unroll
+            for (int c = 0; c < NQ; ++c) {
+                const float4 r4 = *(const float4 *) (red + 4 * c);
+                const float m_new = fmaxf(fmaxf(m_run[c], fmaxf(r4.x, r4.y)), fmaxf(r4.z, r4.w));
+                const float cf = (it <= 0 || m_new == -INFINITY) ? 1.f : exp2f((m_run[c] - m_new) * a.scale_log2e);
+                corr[c] = cf;
+                any_corr |= cf != 1.f;
+                const float pv = (s[c] == -INFINITY) ? 0.f : exp2f((s[c] - m_new) * a.scale_log2e);
+                l_part[c] = l_part[c] * cf + pv;
+                m_run[c] = m_new;
+                // P^T[c][row] (bf16) into the swizzled K-major block
+                const int blk = row >> 6, kcol = row & 63;
+                const uint32_t off = blk * (NQ * 128) + c * 128 + ((((kcol * 2) >> 4) ^ (c & 7)) << 4) + ((kcol * 2) & 15);
+                *(bf16 *) (p_s + off) = __float2bfloat16(pv);
+            }
+            // running-max correction of O^T (previous PV products must have landed)
+            if (it > 0 && ok) {
+                if (!mbar_wait(o_ready, (it - 1) & 1)) { jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 28, it); ok = false; *failed = 1; }
+                tc_fence_after();
+                if (any_corr && ok) {
 #pragma unroll 1
-            for (int m = 0; m < N_LAT_PAIRS; ++m) {
-                const int dim = m * 128 + row;
+                    for (int m = 0; m < N_LAT_PAIRS; ++m)
+#pragma unroll
+                        for (int c = 0; c < NQ; c += 16) {
+                            uint32_t v[16];
+                            tmem_ld16(tm_O + lane_addr + m * NQ + c, v);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * corr[c + j]);
+                            tmem_st16(tm_O + lane_addr + m * NQ + c, v);
+                        }
+                    tmem_st_wait();
+                }
+            }
+            fence_proxy_async();          // P^T stores -> visible to the tensor core's async-proxy reads
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0 && !dry && ok) mbar_arrive(p_ready);
+            asm volatile("bar.sync 1, 128;" ::: "memory");   // red[] reuse in the next tile
+            if (*failed) break;
+            // ---- next tile: the next one of this pass, the first of the next pass with any, or the results ----
+            bool last = dry;
+            if (!dry) {
+                kb += KV_TILE;
+                while (kb >= pass_k1[p]) {
+                    if (++p >= n_pass) { last = true; break; }
+                    kb = pass_k0[p];
+                }
+            }
+            if (last) {
+                // ---- epilogue (in the dry pass without its stores) ----
+                if (!dry) {
+                    if (ok && !mbar_wait(o_ready, (total_tiles - 1) & 1)) { jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 29, 0); ok = false; }
+                    tc_fence_after();
+                    JIB_KS_T(2, 5, 64);
+                }
+                // l per column = sum over the 128 kv lanes: 16 columns of a warp meet in lanes 2 c and 2 c + 1
 #pragma unroll
                 for (int c0 = 0; c0 < NQ; c0 += 16) {
-                    uint32_t v[16];
-                    tmem_ld16(tm_O + lane_addr + m * NQ + c0, v);
-                    tmem_ld_wait();
+                    float x[16];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const int c = c0 + j;
-                        const int t = t0 + (c >> 4), h = hg * 16 + (c & 15);
-                        if (t >= a.T || h >= a.H) continue;
-                        const float o = __uint_as_float(v[j]);
-                        if (a.n_splits > 1) {
-                            a.part_o[(((size_t) t * a.n_splits + sp) * a.H + h) * R + dim] = o;
+                    for (int j = 0; j < 16; ++j) x[j] = l_part[c0 + j];
+#pragma unroll
+                    for (int h = 8; h >= 1; h >>= 1) {
+                        const bool up = lane & (2 * h);
+#pragma unroll
+                        for (int j = 0; j < h; ++j) {
+                            const float give = up ? x[j] : x[j + h], mine = up ? x[j + h] : x[j];
+                            x[j] = mine + __shfl_xor_sync(0xffffffffu, give, 2 * h);
+                        }
+                    }
+                    const float tot = x[0] + __shfl_xor_sync(0xffffffffu, x[0], 1);
+                    if ((lane & 1) == 0) red[(c0 + (lane >> 1)) * 4 + qd] = tot;
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                float inv[NQ];
+                if (a.n_splits == 1) {
+#pragma unroll
+                    for (int c = 0; c < NQ; ++c) {
+                        const float4 r4 = *(const float4 *) (red + 4 * c);
+                        const float l = (r4.x + r4.y) + (r4.z + r4.w);
+                        inv[c] = l > 0.f ? 1.f / l : 0.f;
+                    }
+                }
+                const int n_t = min(QT, a.T - t0), n_h = min(16, a.H - hg * 16);
+                const bool split = a.n_splits > 1;
+                const size_t t_step = (size_t) (split ? a.n_splits : 1) * a.H * R;
+                const size_t at = ((size_t) t0 * (split ? a.n_splits : 1) + (split ? sp : 0)) * a.H * R + (size_t) hg * 16 * R + row;
+#pragma unroll 1
+                for (int m = 0; m < N_LAT_PAIRS; ++m) {
+#pragma unroll
+                    for (int c0 = 0; c0 < NQ; c0 += 16) {
+                        uint32_t v[16];
+                        tmem_ld16(tm_O + lane_addr + m * NQ + c0, v);
+                        tmem_ld_wait();
+                        const size_t base = at + (c0 >> 4) * t_step + m * 128;
+                        const int n_on = dry || !ok || (c0 >> 4) >= n_t ? 0 : n_h;
+                        if (split) {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                if (j < n_on) a.part_o[base + j * R] = __uint_as_float(v[j]);
                         } else {
-                            const float inv = l_tot[c] > 0.f ? 1.f / l_tot[c] : 0.f;
-                            a.o_lat[((size_t) t * a.H + h) * R + dim] = __float2bfloat16(o * inv);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                if (j < n_on) a.o_lat[base + j * R] = __float2bfloat16(__uint_as_float(v[j]) * inv[c0 + j]);
                         }
                     }
                 }
-            }
-            if (a.n_splits > 1 && row < NQ) {
-                // one thread per column publishes (m, l); m is kept in score units * scale (natural-log domain)
-                const int c = row;
-                const int t = t0 + (c >> 4), h = hg * 16 + (c & 15);
-                if (t < a.T && h < a.H) {
-                    const size_t pidx = ((size_t) t * a.n_splits + sp) * a.H + h;
-                    a.part_ml[pidx * 2] = m_run[c] == -INFINITY ? -INFINITY : m_run[c] * a.scale_log2e * 0.6931471805599453f;
-                    a.part_ml[pidx * 2 + 1] = l_tot[c];
+                if (split && !dry && ok && row < NQ) {
+                    // one thread per column publishes (m, l); m is kept in score units * scale (natural-log domain)
+                    const int c = row, t = t0 + (c >> 4), h = hg * 16 + (c & 15);
+                    if (t < a.T && h < a.H) {
+                        float m_c = -INFINITY;
+#pragma unroll
+                        for (int j = 0; j < NQ; ++j)
+                            if (j == c) m_c = m_run[j];
+                        const float4 r4 = *(const float4 *) (red + 4 * c);
+                        const size_t pidx = ((size_t) t * a.n_splits + sp) * a.H + h;
+                        a.part_ml[pidx * 2] = m_c == -INFINITY ? -INFINITY : m_c * a.scale_log2e * 0.6931471805599453f;
+                        a.part_ml[pidx * 2 + 1] = (r4.x + r4.y) + (r4.z + r4.w);
+                    }
                 }
+                if (!dry) break;
+                asm volatile("bar.sync 1, 128;" ::: "memory");      // red[]
+                p = 0;
+                while (pass_k1[p] <= pass_k0[p]) ++p;               // total_tiles > 0: there is one
+                kb = pass_k0[p];
+                pdl_wait();
             }
+            ++it;
         }
     }
 

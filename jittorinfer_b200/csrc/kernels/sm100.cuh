@@ -108,6 +108,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t * bar, uint32_t parity) {
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap * m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
 }
+// The lines of a 2-D tile into L2, nothing else: correct at any time, what is written to them later is what a load will see.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap * m, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(m), "r"(x), "r"(y) : "memory");
+}
 // 3-D tiled load global -> shared, completion on an mbarrier (bytes). No multicast.
 __device__ __forceinline__ void tma_load_3d(void * dst, const CUtensorMap * m, uint64_t * bar, int x, int y, int z) {
     asm volatile(

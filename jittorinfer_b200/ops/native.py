@@ -448,8 +448,9 @@ def mla_attention(q, cache, block_tables, seq_lens, q_start, scale, r, block_siz
     if ATTN_IMPL == "flash" and q.dtype == torch.bfloat16 and r == 512 and D == 576 and block_size == 64 and cache.shape[0] % 64 == 0:
         qt = 2 if prefill else 1
         n_splits = 1 if prefill else attn_splits(T, H)
+        n_splits = max(1, min(n_splits, (block_tables.stride(0) * block_size + 127) // 128))      # a table row names this many 128-row tiles at most
         if window > 0:
-            n_splits = min(n_splits, (window + 63 + 127) // 128)      # a window covers this many 128-row tiles at most
+            n_splits = min(n_splits, (window + 63 + 127) // 128)      # ... and a window covers this many
         part_o = part_ml = None
         if n_splits > 1:
             part_o = torch.empty(T, n_splits, H, r, dtype=torch.float32, device=q.device)
