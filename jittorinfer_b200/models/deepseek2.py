@@ -312,14 +312,19 @@ class DeepSeek2Model:
         else:
             qa, _ = ops.rmsnorm(qkv[:, :nq], L.q_a_norm, hp.rms_eps)
             q = ops.linear(qa, L.w_q_b)
-        if batch.max_q_len > 1 and ops.use_native(q) and q.dtype == torch.bfloat16 and not self.split and \
-                ops.nat().mha_prefill_ok(T, dn, dr, hp.v_head_dim, r, self.block_size, batch.attn_meta):
+        prompts = batch.max_q_len > 1 and ops.use_native(q) and q.dtype == torch.bfloat16 and not self.split
+        sizes = (T, dn, dr, hp.v_head_dim, r, self.block_size, batch.attn_meta)
+        if prompts and ops.nat().mha_prefill_ok(*sizes):
             # prompt chunk: per-head attention over K / V expanded from the latent rows (3.4x fewer FLOPs than the absorbed
             # form); the RoPE part of q is rotated in place, the latent row still goes to the cache for later decode steps
             ops.mla_qkv_post(q, ckv, L.kv_a_norm, hp.rms_eps, self._rope(h.device), batch.positions, batch.slot_mapping, cache_l, None,
                              H, dn, dr, r)
             return ops.nat().mha_prefill(q, cache_l, L.w_kv_b, batch.block_tables, batch.seq_lens, batch.q_start, hp.kq_scale, H,
                                          self.block_size, batch.attn_meta)
+        if prompts and (parts := ops.mla_mixed_split(*sizes)) is not None:
+            return ops.mla_mixed(q, ckv, L.kv_a_norm, hp.rms_eps, self._rope(h.device), batch.positions, batch.slot_mapping, cache_l, L.w_uk,
+                                 L.w_uv, L.w_kv_b, batch.block_tables, batch.seq_lens, batch.q_start, hp.kq_scale, H, dn, dr, r,
+                                 self.block_size, parts)
         q_full = torch.empty(T, H, r + dr, dtype=h.dtype, device=h.device)
         q_nope = ops.mla_qkv_post(q, ckv, L.kv_a_norm, hp.rms_eps, self._rope(h.device), batch.positions,
                                   batch.slot_mapping, cache_l, q_full, H, dn, dr, r)

@@ -376,11 +376,15 @@ class NibalixModel:
         nq = H * (dn + dr)
         q, ckv = qkv[:, :nq], (qkv[:, nq:] if m.kv_from is None else None)
         rows, rope = cache[i], self.rope[(dr, m.rope_base)]
-        if b.max_q_len > 1 and L.w_kv_b is not None and ops.use_native(q) and \
-                ops.nat().mha_prefill_ok(T, dn, dr, m.vdim, r, self.block_size, b.attn_meta, m.window):
+        prompts = b.max_q_len > 1 and L.w_kv_b is not None and ops.use_native(q)
+        sizes = (T, dn, dr, m.vdim, r, self.block_size, b.attn_meta, m.window)
+        if prompts and ops.nat().mha_prefill_ok(*sizes):
             ops.mla_qkv_post(q, ckv, L.kv_norm, self.hp.eps, rope, b.positions, b.slot_mapping, rows, None, H, dn, dr, r, True)
             return ops.nat().mha_prefill(q, rows, L.w_kv_b, b.block_tables, b.seq_lens, b.q_start, m.scale, H, self.block_size, b.attn_meta,
                                          m.window)
+        if prompts and (parts := ops.mla_mixed_split(*sizes)) is not None:
+            return ops.mla_mixed(q, ckv, L.kv_norm, self.hp.eps, rope, b.positions, b.slot_mapping, rows, L.w_uk, L.w_uv, L.w_kv_b,
+                                 b.block_tables, b.seq_lens, b.q_start, m.scale, H, dn, dr, r, self.block_size, parts, m.window, True)
         q_full = torch.empty(T, H, r + dr, dtype=hc.dtype, device=hc.device)
         q_nope = ops.mla_qkv_post(q, ckv, L.kv_norm, self.hp.eps, rope, b.positions, b.slot_mapping, rows, q_full, H, dn, dr, r, True)
         ops.q_absorb(q_nope, L.w_uk, q_full, r)

@@ -95,6 +95,39 @@ def mla_attention(q, cache, block_tables, seq_lens, q_start, scale, r, block_siz
     return ref.mla_attention(q, cache, block_tables, seq_lens, q_start, scale, r, block_size, window)
 
 
+def mla_mixed_split(T: int, dn: int, dr: int, dv: int, r: int, block_size: int, meta, window: int = 0):
+    """For a step whose sequences begin with single tokens (decoding ones, which the scheduler places first) and go on with prompt portions:
+    (number of leading single-token sequences, the others' totals) if the two groups are to take different forms, else None.  One form for
+    all rows is either bad for the prompts (absorbed: every pair of query tokens reads its whole prefix; 2046 prompt tokens beside two
+    contexts of 1025: 288 us a layer) or expands every context for one query row each (whose cost has no bound)."""
+    if meta is None or "q_lens" not in meta:
+        return None
+    q, s = meta["q_lens"], meta["s_lens"]
+    lead = next((i for i, n in enumerate(q) if n != 1), len(q))
+    if lead == 0 or lead == len(q):
+        return None
+    rest = {"total_kv": sum(s[lead:]), "n_q_tiles": sum((n + 127) // 128 for n in q[lead:]),
+            "kv_decode": sum(x for n, x in zip(q[lead:], s[lead:]) if n <= 1), "q_lens": q[lead:], "s_lens": s[lead:]}
+    return (lead, rest) if nat().mha_prefill_ok(T - lead, dn, dr, dv, r, block_size, rest, window) else None
+
+
+def mla_mixed(q, ckv, kv_norm_w, eps, rope_table, positions, slot_mapping, cache, w_uk, w_uv, w_kv_b, block_tables, seq_lens, q_start, scale,
+              n_head, dn, dr, r, block_size, split, window=0, rot_half=False):
+    """Latent attention of a mixed step: the leading single-token rows in the absorbed form, the prompt rows per head
+    (``split`` from ``mla_mixed_split``).  Returns [T, H * dv]."""
+    lead, rest = split
+    post = lambda a, b, q_out: mla_qkv_post(q[a:b], ckv[a:b] if ckv is not None else None, kv_norm_w, eps, rope_table, positions[a:b],      # noqa: E731
+                                            slot_mapping[a:b], cache, q_out, n_head, dn, dr, r, rot_half)
+    q_full = torch.empty(lead, n_head, r + dr, dtype=q.dtype, device=q.device)
+    q_nope = post(0, lead, q_full)
+    post(lead, q.shape[0], None)
+    out = nat().mha_prefill(q, cache, w_kv_b, block_tables[lead:], seq_lens[lead:], q_start[lead:], scale, n_head, block_size, rest, window)
+    q_absorb(q_nope, w_uk, q_full, r)
+    o_lat = mla_attention(q_full, cache, block_tables[:lead], seq_lens[:lead], q_start[:lead + 1], scale, r, block_size, 1, None, window)
+    nat().v_up(o_lat, w_uv, out[:lead])
+    return out
+
+
 def moe_gate(g, w_router, bias, k, n_group, topk_group, scale, norm, sigmoid, n_shared=0, group_top2=False, route=None, pre_norm=None,
              logit_bias=None, shared_gate=False):
     """``w_router`` fp32, or bf16 with bf16 activations (products of exact operands on the tensor cores, fp32 sums).  ``shared_gate``: the last row of ``w_router`` is the shared experts' gate, not an expert: their weight is its sigmoid (``n_shared``

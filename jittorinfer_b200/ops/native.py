@@ -420,11 +420,13 @@ def q_absorb(q_nope, w_ukT, q_out, r):
                  q_out.stride(1), T, q_nope.device)
 
 
-def v_up(o_lat, w_uv):
+def v_up(o_lat, w_uv, out=None):
     """o[t, h*dv:(h+1)*dv] = o_lat[t,h,:] @ w_uv[h]^T with w_uv [H, dv, r]."""
     T, H, r = o_lat.shape
     dv = w_uv.shape[1]
-    out = torch.empty(T, H * dv, dtype=o_lat.dtype, device=o_lat.device)
+    if out is None:
+        out = torch.empty(T, H * dv, dtype=o_lat.dtype, device=o_lat.device)
+    assert out.shape == (T, H * dv) and out.is_contiguous()
     gemm_batched(o_lat.data_ptr(), o_lat.stride(0), o_lat.stride(1), w_uv, out.data_ptr(), H * dv, dv, T, o_lat.device)
     return out
 
