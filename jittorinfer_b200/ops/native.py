@@ -43,7 +43,7 @@ TILE_LIST = os.environ.get("JIB_TILE_LIST", "1") == "1"
 TILE_LIST_MIN_PAIRS = 1024
 # The router launch of a decode batch also applies the RMSNorm of its input ("0": a separate norm launch before it).
 ROUTE_NORM = os.environ.get("JIB_ROUTE_NORM", "1") == "1"
-FUSED_ROUTE_MAX_T = 64
+FUSED_ROUTE_MAX_T = 16                      # past this the separate router's tiles add up in another order (and are faster)
 _route_stash: Dict[tuple, tuple] = {}       # (ids ptr, expert_base, E_local) -> (seg, src, dest) produced by the fused launch
 
 ERRORS = {-1: "unsupported shape/argument", -2: "pointer or stride not 16-byte aligned", -3: "driver entry point missing",
