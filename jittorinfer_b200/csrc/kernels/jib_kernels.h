@@ -114,6 +114,12 @@ JIB_EXPORT int jib_gather_rows(const void * x, const int * src_row, void * out, 
 JIB_EXPORT int jib_moe_gate(const void * g, const float * w_router, const float * bias, const float * logit_bias, float * logits, int * ids,
                             float * wts, int T, int d, int E, int k, int n_group, int topk_group, float scale, int norm, int sigmoid,
                             int n_shared, int group_top2, int shared_gate, void * stream);
+// jib_moe_gate, its gate and jib_moe_permute (over the k + n_shared id columns) as one launch, for T <= 64.  row_wts (or NULL): the weights
+// in sorted order.
+JIB_EXPORT int jib_moe_gate_sort(const void * g, const float * w_router, const float * bias, const float * logit_bias, float * logits, int * ids,
+                                 float * wts, int T, int d, int E, int k, int n_group, int topk_group, float scale, int norm, int sigmoid,
+                                 int n_shared, int group_top2, int shared_gate, int expert_base, int E_local, int * seg, int * src_token,
+                                 int * dest, float * row_wts, void * stream);
 // jib_moe_gate + jib_moe_permute (over the k + n_shared id columns) in one launch, for T <= 64.  counter: one device int that is
 // zero between launches.  norm_w != NULL: the rows of g are RMS-normalised first (as jib_rmsnorm would) and stored to g_out.
 JIB_EXPORT int jib_moe_route_fused(const void * g, const float * w_router, const float * bias, float * logits, int * ids, float * wts,

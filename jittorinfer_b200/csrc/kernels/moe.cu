@@ -319,48 +319,68 @@ int launch_router(const bf16 * g, const float * w_router, float * logits, int T,
     return 0;
 }
 
-// Gating of one token by one warp: softmax/sigmoid over the logits, optional group-limited masking, k rounds of arg-max.
-// prob / sel: MAX_E floats each, gscore: 32 floats, all private to the warp.  Not inlined: the fused router calls it twice
-// (a dry run, then the real one) and both calls must execute the same copy of the code.
+// Gating of one token by one warp: softmax/sigmoid over the logits, optional group-limited masking, k rounds of arg-max.  A lane holds the
+// experts lane, lane + 32, ... in registers; a round is two warp reductions of one instruction each (the largest value, then the lowest
+// expert that has it) instead of ten exchanges and a walk through shared memory.
+// sel: E floats and gscore: 32 floats, private to the warp, with groups only.  Not inlined: callers run it twice (a dry run, then the
+// real one) and both calls must execute the same copy of the code.
+constexpr int GATE_NI = MAX_E / 32;
+
+__device__ __forceinline__ float warp_max(float v) {
+    asm volatile("redux.sync.max.f32 %0, %0, 0xffffffff;" : "+f"(v));
+    return v;
+}
+
 __device__ __noinline__ void gate_token(const float * __restrict__ logits_row, const float * __restrict__ bias, int * __restrict__ ids,
                                            float * __restrict__ wts, int t, int E, int k, int n_group, int topk_group, float scale,
-                                           int norm, int sigmoid, int n_shared, int group_top2, float * prob, float * sel,
-                                           float * gscore, int * ids_copy = nullptr, bool dry = false,
+                                           int norm, int sigmoid, int n_shared, int group_top2, float * sel,
+                                           float * gscore, int * ids_copy = nullptr, float * wts_copy = nullptr, bool dry = false,
                                            const float * __restrict__ logit_bias = nullptr, int shared_gate = 0) {
-    // dry: runs the same instructions on whatever `prob` holds and stores nothing -- a caller that is still waiting for its
+    // dry: runs the same instructions on made-up logits and stores nothing to global memory -- a caller that is still waiting for its
     // inputs uses it to pull this code into the SM's instruction cache ahead of the real call
     const int lane = threadIdx.x & 31;
     const int ld = k + n_shared;
-    if (!dry)
-        for (int e = lane; e < E; e += 32)      // possibly written by other CTAs: from L2
-            prob[e] = __ldcg(logits_row + e) + (logit_bias != nullptr ? logit_bias[e] : 0.f);
-    __syncwarp();
-    // softmax / sigmoid over E (E <= 256 -> 8 per lane)
+    float p[GATE_NI], v[GATE_NI];
     float mx = -FLT_MAX;
-    for (int e = lane; e < E; e += 32) mx = fmaxf(mx, prob[e]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    for (int i = 0; i < GATE_NI; ++i) {
+        const int e = lane + 32 * i;
+        p[i] = 0.f;
+        if (32 * i < E && e < E) {              // possibly written by other CTAs: from L2
+            p[i] = dry ? (float) ((e * 37 + t) & 63) : __ldcg(logits_row + e) + (logit_bias != nullptr ? logit_bias[e] : 0.f);
+            mx = fmaxf(mx, p[i]);
+        }
+    }
+    mx = warp_max(mx);
     float sum = 0.f;
-    for (int e = lane; e < E; e += 32) {
-        const float p = sigmoid ? 1.f / (1.f + expf(-prob[e])) : expf(prob[e] - mx);
-        prob[e] = p;
-        sum += p;
-    }
+#pragma unroll
+    for (int i = 0; i < GATE_NI; ++i)
+        if (32 * i < E && lane + 32 * i < E) {
+            p[i] = sigmoid ? 1.f / (1.f + expf(-p[i])) : expf(p[i] - mx);
+            sum += p[i];
+        }
     sum = warp_sum(sum);
-    __syncwarp();
-    for (int e = lane; e < E; e += 32) {
-        if (!sigmoid) prob[e] = prob[e] / sum;
-        sel[e] = prob[e] + (bias ? bias[e] : 0.f);
+#pragma unroll
+    for (int i = 0; i < GATE_NI; ++i) {
+        const int e = lane + 32 * i;
+        v[i] = -INFINITY;
+        if (32 * i < E && e < E) {
+            if (!sigmoid) p[i] = p[i] / sum;
+            v[i] = p[i] + (bias && !dry ? bias[e] : 0.f);
+        }
     }
-    __syncwarp();
     if (n_group > 1) {
+#pragma unroll
+        for (int i = 0; i < GATE_NI; ++i)
+            if (32 * i < E && lane + 32 * i < E) sel[lane + 32 * i] = v[i];
+        __syncwarp();
         const int gs = E / n_group;
         if (lane < n_group) {
             // a group's score: its best expert (DeepSeek-V2) or the sum of its two best (DeepSeek-V3)
             float m = -FLT_MAX, m2 = -FLT_MAX;
             for (int j = 0; j < gs; ++j) {
-                const float v = sel[lane * gs + j];
-                if (v > m) { m2 = m; m = v; } else if (v > m2) { m2 = v; }
+                const float x = sel[lane * gs + j];
+                if (x > m) { m2 = m; m = x; } else if (x > m2) { m2 = x; }
             }
             gscore[lane] = (group_top2 && gs >= 2) ? m + m2 : m;
         }
@@ -374,45 +394,46 @@ __device__ __noinline__ void gate_token(const float * __restrict__ logits_row, c
                 for (int j = 0; j < gs; ++j) sel[lane * gs + j] = -INFINITY;
         }
         __syncwarp();
+#pragma unroll
+        for (int i = 0; i < GATE_NI; ++i)
+            if (32 * i < E && lane + 32 * i < E) v[i] = sel[lane + 32 * i];
+        __syncwarp();
     }
     // k rounds of warp arg-max (ties -> lower expert id); lane `round` keeps that round's pick
     float wsum = 0.f, my_w = 0.f;
     int my_id = 0;
     for (int round = 0; round < k; ++round) {
         float bv = -INFINITY;
-        int bi = 0x7fffffff;
-        for (int e = lane; e < E; e += 32) {
-            const float v = sel[e];
-            if (v > bv || (v == bv && e < bi)) { bv = v; bi = e; }
-        }
+        unsigned bi = 0x7fffffffu;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-        }
-        if (bi >= E) bi = 0;     // a -inf that was already masked can only be re-picked when fewer than k experts are eligible
-        const float p = prob[bi];
-        if (lane == round) { my_id = bi; my_w = p; }
-        if (lane == 0) sel[bi] = -INFINITY;
-        wsum += p;
-        __syncwarp();
+        for (int i = 0; i < GATE_NI; ++i)
+            if (32 * i < E && lane + 32 * i < E && (v[i] > bv || (v[i] == bv && bi == 0x7fffffffu))) { bv = v[i]; bi = lane + 32 * i; }
+        const float top = warp_max(bv);
+        unsigned pick = __reduce_min_sync(0xffffffffu, bv == top ? bi : 0x7fffffffu);
+        if (pick >= (unsigned) E) pick = 0;     // no number among the scores; a masked -inf is re-picked when fewer than k experts are eligible
+        float w = 0.f;
+#pragma unroll
+        for (int i = 0; i < GATE_NI; ++i)
+            if ((int) (pick >> 5) == i) {
+                w = p[i];
+                if ((int) (pick & 31) == lane) v[i] = -INFINITY;
+            }
+        w = __shfl_sync(0xffffffffu, w, pick & 31);
+        if (lane == round) { my_id = (int) pick; my_w = w; }
+        wsum += w;
     }
-    if (lane < k) {
-        float w = my_w;
-        if (norm) w /= wsum;
-        if (!dry) {
-            ids[(size_t) t * ld + lane] = my_id;
-            wts[(size_t) t * ld + lane] = w * scale;
-        }
-        if (ids_copy != nullptr) ids_copy[t * ld + lane] = my_id;
-    } else if (lane < ld) {
+    if (lane < ld) {
         // shared experts ride along as always-selected experts E, E+1, ... with weight 1, or that of their gate
+        const bool routed = lane < k;
+        const int id = routed ? my_id : E + (lane - k);
+        float w = routed ? (norm ? my_w / wsum : my_w) * scale : 1.f;
+        if (!routed && shared_gate && !dry) w = 1.f / (1.f + expf(-__ldcg(logits_row + E)));
         if (!dry) {
-            ids[(size_t) t * ld + lane] = E + (lane - k);
-            wts[(size_t) t * ld + lane] = shared_gate ? 1.f / (1.f + expf(-__ldcg(logits_row + E))) : 1.f;
+            ids[(size_t) t * ld + lane] = id;
+            wts[(size_t) t * ld + lane] = w;
         }
-        if (ids_copy != nullptr) ids_copy[t * ld + lane] = E + (lane - k);
+        if (ids_copy != nullptr) ids_copy[t * ld + lane] = id;
+        if (wts_copy != nullptr) wts_copy[t * ld + lane] = w;
     }
 }
 
@@ -423,21 +444,16 @@ __global__ void __launch_bounds__(32) moe_gate_kernel(const float * __restrict__
                                                       int group_top2, const float * __restrict__ logit_bias, int shared_gate, int warm) {
     JIB_KS(10, 0);
     PDL_TRIGGER_TOP();
-    __shared__ float prob[MAX_E];
     __shared__ float sel[MAX_E];
     __shared__ float gscore[32];
     const int t = blockIdx.x;
-    if (warm) {
-        for (int e = threadIdx.x & 31; e < MAX_E; e += 32) prob[e] = (float) ((e * 37 + t) & 63);
-        __syncwarp();
-        gate_token(nullptr, bias == nullptr ? nullptr : (const float *) prob, nullptr, nullptr, 0, E, k, n_group, topk_group, scale, norm,
-                   sigmoid, n_shared, group_top2, prob, sel, gscore, nullptr, true);
-        __syncwarp();
-    }
+    if (warm)
+        gate_token(nullptr, bias, nullptr, nullptr, 0, E, k, n_group, topk_group, scale, norm, sigmoid, n_shared, group_top2, sel, gscore,
+                   nullptr, nullptr, true);
     pdl_wait();      // inputs come from earlier kernels; nothing is written before this point
     JIB_KS(10, 1);
     gate_token(logits + (size_t) t * (E + shared_gate), bias, ids, wts, t, E, k, n_group, topk_group, scale, norm, sigmoid, n_shared, group_top2,
-               prob, sel, gscore, nullptr, false, logit_bias, shared_gate);
+               sel, gscore, nullptr, nullptr, false, logit_bias, shared_gate);
     JIB_KS(10, 9);
 }
 
@@ -519,6 +535,85 @@ __device__ __noinline__ void sort_pairs(const int * __restrict__ ids, int n, int
     }
 }
 
+// The same for at most SORT_MATCH_MAX pairs whose ids lie in shared memory: every warp ranks 32 pairs at a time among themselves with one
+// match, the experts add up over those runs of 32, and every pair knows its row: one look at the ids, where the walk above looks at all ids
+// twice per expert.
+// cnt: n / 32 x E_local numbers; at least n / 128 warps.
+constexpr int SORT_MATCH_MAX = 4096, SORT_RUNS = 4;
+__device__ __noinline__ void sort_match(const int * ids_s, int n, int k, int expert_base, int E_local, int * __restrict__ seg,
+                                        int * __restrict__ src_token, int * __restrict__ dest, unsigned short * cnt, int * count, int * offs,
+                                        bool dry, int * __restrict__ active, const float * wts, float * __restrict__ row_wts) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, runs = (n + 31) / 32;
+    for (int x = threadIdx.x; x < runs * E_local; x += blockDim.x) cnt[x] = 0;
+    __syncthreads();
+    int le[SORT_RUNS], rank[SORT_RUNS];
+#pragma unroll
+    for (int r = 0; r < SORT_RUNS; ++r) {
+        const int c = warp + r * nw, i = c * 32 + lane;
+        if (c < runs) {
+            le[r] = i < n ? ids_s[i] - expert_base : -1;
+            if (le[r] < 0 || le[r] >= E_local) le[r] = -1;
+            const unsigned same = __match_any_sync(0xffffffffu, le[r]);
+            rank[r] = __popc(same & ((1u << lane) - 1));
+            if (le[r] >= 0 && rank[r] == 0) cnt[c * E_local + le[r]] = (unsigned short) __popc(same);
+        }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < E_local; e += blockDim.x) {
+        int run = 0;
+        for (int c = 0; c < runs; ++c) {
+            const int v = cnt[c * E_local + e];
+            cnt[c * E_local + e] = (unsigned short) run;
+            run += v;
+        }
+        count[e] = run;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        // exclusive prefix over the experts, and the experts that have rows, in order, then -1
+        int run = 0, n_act = 0;
+        for (int e0 = 0; e0 < E_local; e0 += 32) {
+            const int e = e0 + lane, c = e < E_local ? count[e] : 0;
+            int inc = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += v;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, c > 0);
+            if (e < E_local) {
+                offs[e] = run + inc - c;
+                if (!dry) {
+                    seg[e] = run + inc - c;
+                    if (c > 0) active[n_act + __popc(m & ((1u << lane) - 1))] = e;
+                }
+            }
+            run += __shfl_sync(0xffffffffu, inc, 31);
+            n_act += __popc(m);
+        }
+        if (lane == 0) offs[E_local] = run;
+        if (!dry) {
+            if (lane == 0) seg[E_local] = run;
+            for (int i = n_act + lane; i < E_local; i += 32) active[i] = -1;
+        }
+    }
+    __syncthreads();
+    if (!dry)
+        for (int i = offs[E_local] + threadIdx.x; i < n; i += blockDim.x) src_token[i] = -1;      // rows no local expert owns
+#pragma unroll
+    for (int r = 0; r < SORT_RUNS; ++r) {
+        const int c = warp + r * nw, i = c * 32 + lane;
+        if (c < runs && i < n && !dry) {
+            const int row = le[r] < 0 ? -1 : offs[le[r]] + cnt[c * E_local + le[r]] + rank[r];
+            dest[i] = row;
+            if (row >= 0) {
+                src_token[row] = i / k;
+                if (row_wts != nullptr) row_wts[row] = wts[i];
+            }
+        }
+    }
+}
+
 __global__ void __launch_bounds__(1024) moe_permute_kernel(const int * __restrict__ ids, int n, int k, int expert_base, int E_local,
                                                           int * __restrict__ seg, int * __restrict__ src_token, int * __restrict__ dest,
                                                           int warm, int * __restrict__ active, const float * __restrict__ wts,
@@ -528,20 +623,65 @@ __global__ void __launch_bounds__(1024) moe_permute_kernel(const int * __restric
     __shared__ int count[MAX_E + 1];
     __shared__ int offs[MAX_E + 1];
     __shared__ int ids_s[SORT_SMEM_MAX];
-    if (warm) {
+    extern __shared__ unsigned short cnt_s[];
+    const bool few = n <= SORT_MATCH_MAX;
+    if (warm && few) {
         for (int i = threadIdx.x; i < 32; i += blockDim.x) ids_s[i] = expert_base + (i % max(E_local, 1));
         __syncthreads();
-        sort_pairs(ids_s, min(n, 32), k, expert_base, E_local, nullptr, nullptr, nullptr, count, offs, true);
+        sort_match(ids_s, min(n, 32), k, expert_base, E_local, nullptr, nullptr, nullptr, cnt_s, count, offs, true, nullptr, nullptr, nullptr);
         __syncthreads();
     }
     pdl_wait();      // inputs come from earlier kernels; nothing is written before this point
     JIB_KS(11, 1);
-    if (n <= SORT_SMEM_MAX) {
+    if (few) {
         for (int i = threadIdx.x; i < n; i += blockDim.x) ids_s[i] = ids[i];
         __syncthreads();
+        sort_match(ids_s, n, k, expert_base, E_local, seg, src_token, dest, cnt_s, count, offs, false, active, wts, row_wts);
+    } else {
+        sort_pairs(ids, n, k, expert_base, E_local, seg, src_token, dest, count, offs, false, active, wts, row_wts);
     }
-    sort_pairs(n <= SORT_SMEM_MAX ? ids_s : ids, n, k, expert_base, E_local, seg, src_token, dest, count, offs, false, active, wts, row_wts);
     JIB_KS(11, 9);
+}
+
+// Gating and expert sort of up to GATE_SORT_T tokens in one CTA, a warp per token (two, past 32): what the second kernel would read back
+// are ids in shared memory, and one launch of the chain is gone.  From the router's end to the sort's inside a decode graph: 4 tokens, 8.2 ->
+// 5.8 us, 64 tokens (64 + 2 experts, 8 choices) 17.7 -> 12.7 us.  Past 64 tokens a warp would gate three and more in a row, while one CTA
+// per token gates them side by side.
+constexpr int GATE_SORT_T = 64;
+__global__ void __launch_bounds__(1024) moe_gate_sort_kernel(const float * __restrict__ logits, const float * __restrict__ bias,
+                                                            const float * __restrict__ logit_bias, int * __restrict__ ids, float * __restrict__ wts,
+                                                            int T, int E, int k, int n_group, int topk_group, float scale, int norm, int sigmoid,
+                                                            int n_shared, int group_top2, int shared_gate, int expert_base, int E_local,
+                                                            int * __restrict__ seg, int * __restrict__ src_token, int * __restrict__ dest,
+                                                            float * __restrict__ row_wts, int warm) {
+    JIB_KS(10, 0);
+    PDL_TRIGGER_TOP();
+    __shared__ int count[MAX_E + 1];
+    __shared__ int offs[MAX_E + 1];
+    __shared__ float gscore[32][32];
+    extern __shared__ __align__(16) uint8_t gs_smem[];
+    const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5, ld = k + n_shared, n = T * ld;
+    int * ids_s = (int *) gs_smem;
+    float * wts_s = (float *) (ids_s + n);
+    float * sel = wts_s + n + (n_group > 1 ? warp * E : 0);
+    unsigned short * cnt = (unsigned short *) (wts_s + n + (n_group > 1 ? nw * E : 0));
+    if (warm) {
+        if (warp < T)
+            gate_token(nullptr, bias, nullptr, nullptr, warp, E, k, n_group, topk_group, scale, norm, sigmoid, n_shared, group_top2, sel, gscore[warp],
+                       ids_s, wts_s, true);
+        __syncthreads();
+        sort_match(ids_s, ld, ld, expert_base, E_local, nullptr, nullptr, nullptr, cnt, count, offs, true, nullptr, nullptr, nullptr);
+        __syncthreads();
+    }
+    pdl_wait();      // inputs come from earlier kernels; nothing is written before this point
+    JIB_KS(10, 1);
+    for (int t = warp; t < T; t += nw)
+        gate_token(logits + (size_t) t * (E + shared_gate), bias, ids, wts, t, E, k, n_group, topk_group, scale, norm, sigmoid, n_shared, group_top2,
+                   sel, gscore[warp], ids_s, wts_s, false, logit_bias, shared_gate);
+    __syncthreads();         // ids of all tokens are in shared memory
+    JIB_KS(10, 2);
+    sort_match(ids_s, n, ld, expert_base, E_local, seg, src_token, dest, cnt, count, offs, false, seg + E_local + 1, wts_s, row_wts);
+    JIB_KS(10, 9);
 }
 
 // ---- the same sort for large n (prefill) on many CTAs: histogram per 1024-pair chunk, scan, stable scatter ----------
@@ -655,7 +795,6 @@ __global__ void __launch_bounds__(GATE_NT) moe_route_fused_kernel(const bf16 * _
     __shared__ float red[GATE_NT / 32][GATE_TG];
     __shared__ float inv_s[GATE_TG];
     __shared__ int s_last;
-    __shared__ float prob_s[GATE_NT / 32][MAX_E];
     __shared__ float sel_s[GATE_NT / 32][MAX_E];
     __shared__ float gscore_s[GATE_NT / 32][32];
     __shared__ int ids_s[ROUTE_MAX_T * 32];      // k + n_shared <= 32 columns
@@ -665,10 +804,8 @@ __global__ void __launch_bounds__(GATE_NT) moe_route_fused_kernel(const bf16 * _
     if (warm) {
         // While the previous kernel is still running: walk the gating and sorting code once on scratch values, storing
         // nothing, so that whichever CTA turns out to be last finds that code in its SM's instruction cache.
-        for (int e = threadIdx.x & 31; e < MAX_E; e += 32) prob_s[warp][e] = (float) ((e * 37 + warp) & 63);
-        __syncwarp();
-        gate_token(nullptr, bias == nullptr ? nullptr : (const float *) prob_s[warp], nullptr, nullptr, 0, E, k, n_group, topk_group, scale,
-                   norm, sigmoid, n_shared, group_top2, prob_s[warp], sel_s[warp], gscore_s[warp], ids_s, true);
+        gate_token(nullptr, bias, nullptr, nullptr, 0, E, k, n_group, topk_group, scale, norm, sigmoid, n_shared, group_top2, sel_s[warp],
+                   gscore_s[warp], ids_s, nullptr, true);
         __syncthreads();
         sort_pairs(ids_s, k + n_shared, k + n_shared, expert_base, E_local, nullptr, nullptr, nullptr, count, offs, true);
         __syncthreads();
@@ -690,7 +827,7 @@ __global__ void __launch_bounds__(GATE_NT) moe_route_fused_kernel(const bf16 * _
     // ---- gating: warp w takes tokens w, w + 8, ... ----
     for (int t = warp; t < T; t += GATE_NT / 32) {
         gate_token(logits + (size_t) t * E, bias, ids, wts, t, E, k, n_group, topk_group, scale, norm, sigmoid, n_shared, group_top2,
-                   prob_s[warp], sel_s[warp], gscore_s[warp], ids_s);
+                   sel_s[warp], gscore_s[warp], ids_s);
         __syncwarp();
     }
     __syncthreads();         // ids of all tokens are in shared memory
@@ -924,18 +1061,43 @@ JIB_TL_DEFINE_SETTER(moe)
 
 extern "C" {
 
+static bool gate_args_ok(int E, int k, int n_group, int n_shared) {
+    return E <= MAX_E && k + n_shared <= 32 && n_shared >= 0 && k <= E && n_group <= 32 && !(n_group > 1 && E % n_group);
+}
+
+static int router_of(const void * g, const float * w_router, float * logits, int T, int d, int E, void * stream) {
+    if (g == nullptr) return 0;
+    if (d % 8 || d > GATE_MAXC * GATE_NT * 8) return JIB_E_ARG;
+    return launch_router((const bf16 *) g, w_router, logits, T, d, E, (cudaStream_t) stream);
+}
+
 int jib_moe_gate(const void * g, const float * w_router, const float * bias, const float * logit_bias, float * logits, int * ids, float * wts,
                  int T, int d, int E, int k, int n_group, int topk_group, float scale, int norm, int sigmoid, int n_shared, int group_top2,
                  int shared_gate, void * stream) {
     if (T <= 0) return 0;
     shared_gate = shared_gate ? 1 : 0;
-    if (E > MAX_E || k + n_shared > 32 || n_shared < 0 || k > E || n_group > 32 || (n_group > 1 && E % n_group)) return JIB_E_ARG;
-    if (g != nullptr) {
-        if (d % 8 || d > GATE_MAXC * GATE_NT * 8) return JIB_E_ARG;
-        if (int rc = launch_router((const bf16 *) g, w_router, logits, T, d, E + shared_gate, (cudaStream_t) stream)) return rc;
-    }
+    if (!gate_args_ok(E, k, n_group, n_shared)) return JIB_E_ARG;
+    if (int rc = router_of(g, w_router, logits, T, d, E + shared_gate, stream)) return rc;
     JIB_LAUNCH((moe_gate_kernel), T, 32, 0, (cudaStream_t) stream, logits, bias, ids, wts, E, k, n_group, topk_group, scale, norm, sigmoid, n_shared, group_top2,
                logit_bias, shared_gate, jib::warm_for(T));
+    return launched();
+}
+
+// jib_moe_gate and jib_moe_permute over its k + n_shared columns, the gate and the sort in one launch; T <= 64.  row_wts (or NULL)
+// [T * (k + n_shared)]: the weights in sorted order.
+int jib_moe_gate_sort(const void * g, const float * w_router, const float * bias, const float * logit_bias, float * logits, int * ids, float * wts,
+                      int T, int d, int E, int k, int n_group, int topk_group, float scale, int norm, int sigmoid, int n_shared, int group_top2,
+                      int shared_gate, int expert_base, int E_local, int * seg, int * src_token, int * dest, float * row_wts, void * stream) {
+    if (T <= 0) return 0;
+    shared_gate = shared_gate ? 1 : 0;
+    if (!gate_args_ok(E, k, n_group, n_shared) || T > GATE_SORT_T || E_local < 1 || E_local > MAX_E) return JIB_E_ARG;
+    if (int rc = router_of(g, w_router, logits, T, d, E + shared_gate, stream)) return rc;
+    const int nw = T < 4 ? 4 : T > 32 ? 32 : T, n = T * (k + n_shared);       // n / 32 <= T runs: at most two per warp
+    const int smem = n * 8 + (n_group > 1 ? nw * E * 4 : 0) + (n + 31) / 32 * E_local * 2;
+    static std::atomic<unsigned char> attr_done[jib::MAX_DEVICES];
+    if (!jib::ensure_dyn_smem(moe_gate_sort_kernel, 96 * 1024, attr_done)) return JIB_E_LAUNCH;
+    JIB_LAUNCH((moe_gate_sort_kernel), 1, nw * 32, smem, (cudaStream_t) stream, logits, bias, logit_bias, ids, wts, T, E, k, n_group, topk_group, scale, norm,
+               sigmoid, n_shared, group_top2, shared_gate, expert_base, E_local, seg, src_token, dest, row_wts, jib::warm_for(T));
     return launched();
 }
 
@@ -960,7 +1122,10 @@ int jib_moe_permute(const int * ids, int T, int k, int expert_base, int E_local,
                     float * row_wts, void * stream) {
     if (T <= 0) return 0;
     if (E_local > MAX_E || (row_wts != nullptr && wts == nullptr)) return JIB_E_ARG;
-    JIB_LAUNCH((moe_permute_kernel), 1, 1024, 0, (cudaStream_t) stream, ids, T * k, k, expert_base, E_local, seg, src_token, dest,
+    const int smem = T * k <= SORT_MATCH_MAX ? (T * k + 31) / 32 * E_local * 2 : 0;
+    static std::atomic<unsigned char> attr_done[jib::MAX_DEVICES];
+    if (!jib::ensure_dyn_smem(moe_permute_kernel, SORT_MATCH_MAX / 32 * MAX_E * 2, attr_done)) return JIB_E_LAUNCH;
+    JIB_LAUNCH((moe_permute_kernel), 1, 1024, smem, (cudaStream_t) stream, ids, T * k, k, expert_base, E_local, seg, src_token, dest,
                jib::warm_for(T), seg + E_local + 1, wts, row_wts);
     return launched();
 }

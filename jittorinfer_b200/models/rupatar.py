@@ -428,7 +428,7 @@ class RupatarModel:
 
     def _ff(self, L: _Layer, m: Experts, h: torch.Tensor) -> Dict[str, Any]:
         """The feed-forward's part of ``ops.scaled_update``'s arguments."""
-        ids, wts = ops.moe_gate(h, L.router, None, m.top, 1, 1, 1.0, False, True, L.n_merged)
+        ids, wts = ops.moe_gate(h, L.router, None, m.top, 1, 1, 1.0, False, True, L.n_merged, route=(0, L.w_up_exps.shape[0]))
         y, dest = ops.moe_routed(h, ids, wts, None, L.w_up_exps, L.w_down_exps)
         out: Dict[str, Any] = {"moe": (y, dest, None)}
         if m.shared is not None and not L.n_merged:

@@ -44,6 +44,7 @@ TILE_LIST_MIN_PAIRS = 1024
 # The router launch of a decode batch also applies the RMSNorm of its input ("0": a separate norm launch before it).
 ROUTE_NORM = os.environ.get("JIB_ROUTE_NORM", "1") == "1"
 FUSED_ROUTE_MAX_T = 16                      # past this the separate router's tiles add up in another order (and are faster)
+GATE_SORT_MAX_T = 64                        # gate and expert sort as one launch: every token is a warp of one CTA
 _route_stash: Dict[tuple, tuple] = {}       # (ids ptr, expert_base, E_local) -> (seg, src, dest) produced by the fused launch
 
 ERRORS = {-1: "unsupported shape/argument", -2: "pointer or stride not 16-byte aligned", -3: "driver entry point missing",
@@ -140,6 +141,7 @@ def load():
     sig("jib_kv_block_copy", vp, ll, i, ip, ip, i, i, vp)
     sig("jib_gather_rows", vp, ip, vp, i, i, i, vp)
     sig("jib_moe_gate", vp, fp, fp, fp, fp, ip, fp, i, i, i, i, i, i, f, i, i, i, i, i, vp)
+    sig("jib_moe_gate_sort", vp, fp, fp, fp, fp, ip, fp, i, i, i, i, i, i, f, i, i, i, i, i, i, i, ip, ip, ip, fp, vp)
     sig("jib_moe_permute", ip, i, i, i, i, ip, ip, ip, fp, fp, vp)
     sig("jib_moe_route_fused", vp, fp, fp, fp, ip, fp, ip, ip, ip, ip, i, i, i, i, i, i, f, i, i, i, i, i, i, fp, f, vp, vp)
     sig("jib_moe_permute_multi", ip, i, i, i, i, ip, ip, ip, ip, fp, fp, vp)
@@ -551,8 +553,8 @@ def mha_prefill(q, cache, w_kv_b, block_tables, seq_lens, q_start, scale, n_head
 # ---- MoE -----------------------------------------------------------------------------------------
 def moe_gate(g, w_router, bias, k, n_group, topk_group, scale, norm, sigmoid, n_shared=0, group_top2=False, route=None,
              pre_norm=None, logit_bias=None, shared_gate=False):
-    """``route=(expert_base, E_local)``: the caller will sort these ids by local expert next (``moe_permute``); for decode
-    batches both steps then run as one launch and ``moe_permute`` picks the result up.
+    """``route=(expert_base, E_local)``: the caller will sort these ids by local expert next (``moe_permute``, ``moe_routed``); for decode
+    batches the gate and the sort then run as one launch, whose result travels with ``ids``.
     ``pre_norm=(weight, eps)``: ``g`` holds un-normalised rows; returns (ids, wts, rmsnorm(g) * weight), the norm done by
     the router launch itself for decode batches."""
     T, d = g.shape
@@ -592,10 +594,33 @@ def moe_gate(g, w_router, bias, k, n_group, topk_group, scale, norm, sigmoid, n_
         gemm(g, w_router, out=logits)
     elif not own:
         torch.matmul(g.float(), w_router.T, out=logits)
+    if route is not None and 0 < T <= GATE_SORT_MAX_T and not ids.is_inference():
+        expert_base, E_local = route
+        n = T * (k + n_shared)
+        seg = torch.empty(2 * E_local + 1, dtype=torch.int32, device=g.device)[:E_local + 1]     # + room for the list of experts hit
+        src, dest, row_wts = torch.empty(n, dtype=torch.int32, device=g.device), torch.empty_like(ids), torch.empty(n, dtype=torch.float32, device=g.device)
+        _ck(load().jib_moe_gate_sort(g.data_ptr() if own else None, w_router.data_ptr(), _p(bias), _p(logit_bias), logits.data_ptr(), ids.data_ptr(),
+                                     wts.data_ptr(), T, d, E, k, n_group, topk_group, float(scale), int(norm), int(sigmoid), n_shared, int(group_top2),
+                                     int(shared_gate), expert_base, E_local, seg.data_ptr(), src.data_ptr(), dest.data_ptr(), row_wts.data_ptr(),
+                                     _stream()), "moe_gate_sort")
+        ids.sorted_pairs = (expert_base, E_local, ids._version, seg, src, dest)
+        wts.sorted_pairs = (ids.data_ptr(), wts._version, row_wts)
+        return (ids, wts) + ((g,) if pre_norm is not None else ()) + ((logits[:, E],) if shared_gate else ())
     _ck(load().jib_moe_gate(g.data_ptr() if own else None, w_router.data_ptr(), _p(bias), _p(logit_bias), logits.data_ptr(), ids.data_ptr(), wts.data_ptr(), T, d,
                             E, k, n_group, topk_group, float(scale), int(norm), int(sigmoid), n_shared, int(group_top2), int(shared_gate), _stream()),
         "moe_gate")
     return (ids, wts) + ((g,) if pre_norm is not None else ()) + ((logits[:, E],) if shared_gate else ())
+
+
+def _sorted_by_gate(ids, expert_base, E_local):
+    """(seg, src, dest) of ids that a gate launch sorted for these experts and that nobody has written to since, else None."""
+    r = getattr(ids, "sorted_pairs", None)
+    return r[3:] if r is not None and r[:3] == (expert_base, E_local, ids._version) else None
+
+
+def _row_weights_of_gate(ids, wts):
+    r = getattr(wts, "sorted_pairs", None)
+    return r[2] if r is not None and r[:2] == (ids.data_ptr(), wts._version) else None
 
 
 def moe_permute(ids, expert_base, E_local, wts=None, row_wts=None):
@@ -605,6 +630,9 @@ def moe_permute(ids, expert_base, E_local, wts=None, row_wts=None):
     hit = _route_stash.pop((ids.data_ptr(), expert_base, E_local), None)
     if hit is not None and hit[3] is ids and row_wts is None:          # the fused router launch already sorted exactly these ids
         return hit[0], hit[1], hit[2]
+    hit = _sorted_by_gate(ids, expert_base, E_local)
+    if hit is not None and row_wts is None:
+        return hit
     seg = torch.empty(2 * E_local + 1, dtype=torch.int32, device=dev)[:E_local + 1]       # + room for the list of experts hit
     src = torch.empty(T * k, dtype=torch.int32, device=dev)
     dest = torch.empty(T, k, dtype=torch.int32, device=dev)
@@ -667,8 +695,12 @@ def moe_routed(x, ids, wts, wg, wu, wd, expert_base=0, n_expert=None):
     epilogue gelu(weight of the row * product).  Returns (y [T*k, d] in sorted order, dest [T,k])."""
     T, k = ids.shape
     E_local = wu.shape[0]
-    fn = None if wg is not None else torch.empty(T * k, dtype=torch.float32, device=x.device)
-    seg, src, dest = moe_permute(ids, expert_base, E_local, wts if fn is not None else None, fn)
+    fn = _row_weights_of_gate(ids, wts) if wg is None and _sorted_by_gate(ids, expert_base, E_local) is not None else None
+    if fn is not None or wg is not None:
+        seg, src, dest = moe_permute(ids, expert_base, E_local)
+    else:
+        fn = torch.empty(T * k, dtype=torch.float32, device=x.device)
+        seg, src, dest = moe_permute(ids, expert_base, E_local, wts, fn)
     if fn is not None:
         wg, wu = wu, None
     if not grouped_tma_ok(x, wg):                  # fp32 operands, or rows TMA cannot address

@@ -1,0 +1,97 @@
+"""Gate and expert sort of up to 64 tokens as one launch, and the sort by matching: against the separate launches and a stable sort."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture(scope="module")
+def nat():
+    from jittorinfer_b200.ops import native
+    native.load()
+    yield native
+    torch.cuda.synchronize()
+    native.check_status()
+
+
+def check_sort(ids, base, E_local, seg, src, dest):
+    T, k = ids.shape
+    flat = ids.flatten().long().cpu() - base
+    ok = (flat >= 0) & (flat < E_local)
+    order = torch.sort(torch.where(ok, flat, torch.full_like(flat, E_local)), stable=True).indices
+    n = int(ok.sum())
+    want = torch.full_like(flat, -1)
+    want[order[:n]] = torch.arange(n)
+    assert torch.equal(dest.flatten().cpu().long(), want)
+    assert torch.equal(src.cpu().long()[:n], order[:n] // k) and bool((src[n:] == -1).all())
+    counts = torch.bincount(flat[ok], minlength=E_local)
+    assert torch.equal(seg.cpu().long(), torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)]))
+    active = torch.full((E_local,), -1)
+    hit = torch.nonzero(counts).flatten()
+    active[:len(hit)] = hit
+    room = torch.as_strided(seg, (E_local,), (1,), seg.storage_offset() + E_local + 1)
+    assert torch.equal(room.cpu().long(), active)
+    return order[:n]
+
+
+# warps with no, one and two tokens; runs of 32 pairs that end within, at and past a warp; experts below, at and past a lane's registers
+@pytest.mark.parametrize("T", [1, 3, 4, 5, 31, 32, 33, 64, 65])
+@pytest.mark.parametrize("E,k,n_shared,n_group,topk_group,top2,sigmoid,norm,base,E_local",
+                         [(64, 6, 2, 1, 1, False, False, False, 0, 66), (160, 6, 0, 8, 3, False, False, False, 40, 20),
+                          (256, 8, 0, 8, 4, True, True, True, 0, 256), (7, 7, 1, 1, 1, False, True, True, 0, 8), (33, 31, 1, 1, 1, False, False, True, 3, 5)])
+def test_one_launch(nat, T, E, k, n_shared, n_group, topk_group, top2, sigmoid, norm, base, E_local):
+    gen = torch.Generator(device=DEV).manual_seed(T + E)
+    x = torch.randn(T, 512, generator=gen, device=DEV).bfloat16()
+    w = torch.randn(E, 512, generator=gen, device=DEV) * 0.05
+    if n_group == 1:
+        w[E // 2:] = w[:E - E // 2].clone()                                   # choices between experts of equal score
+    bias = torch.rand(E, generator=gen, device=DEV) * 0.01 if sigmoid and n_group > 1 else None
+    lb = torch.randn(E, generator=gen, device=DEV) if n_group == 1 and E != 64 else None
+    args = (x, w, bias, k, n_group, topk_group, 2.5, norm, sigmoid, n_shared, top2)
+    ids0, wts0 = nat.moe_gate(*args, logit_bias=lb)
+    for _ in range(2):
+        ids, wts = nat.moe_gate(*args, route=(base, E_local), logit_bias=lb)
+    assert torch.equal(ids, ids0) and torch.equal(wts, wts0)
+    seg, src, dest = nat.moe_permute(ids, base, E_local)
+    order = check_sort(ids, base, E_local, seg, src, dest)
+    if T <= nat.GATE_SORT_MAX_T:
+        assert src.data_ptr() == ids.sorted_pairs[4].data_ptr()               # the gate's own
+        rows = nat._row_weights_of_gate(ids, wts)
+        assert torch.equal(rows[:len(order)].cpu(), wts.flatten().cpu()[order])
+        assert nat.moe_permute(ids, base, E_local - 1)[1].data_ptr() != src.data_ptr()
+        ids += 0                                                              # written to: sorted anew
+        assert nat._sorted_by_gate(ids, base, E_local) is None
+        wts.mul_(2)
+        assert nat._row_weights_of_gate(ids, wts) is None
+    with torch.inference_mode():                                              # no version counters: the two launches
+        ids, wts = nat.moe_gate(*args, route=(base, E_local), logit_bias=lb)
+        assert torch.equal(ids, ids0) and not hasattr(ids, "sorted_pairs")
+
+
+def test_no_numbers_and_infinities(nat):
+    """Scores that are all NaN pick expert 0; fewer numbers than choices re-pick the lowest masked one."""
+    E, k = 40, 4
+    logits = torch.zeros(3, E, device=DEV)
+    logits[0] = float("nan")
+    logits[1] = float("-inf")
+    logits[1, 7] = 1.0
+    logits[2, 33] = logits[2, 5] = 3.0
+    ids = torch.empty(3, k, dtype=torch.int32, device=DEV)
+    wts = torch.empty(3, k, device=DEV)
+    nat._ck(nat.load().jib_moe_gate(None, None, None, None, logits.data_ptr(), ids.data_ptr(), wts.data_ptr(), 3, 8, E, k, 1, 1, 1.0, 0, 0, 0, 0, 0,
+                                    nat._stream()), "moe_gate")
+    assert ids[0].tolist() == [0, 0, 0, 0]
+    assert ids[1].tolist() == [7, 0, 1, 2] and wts[1].tolist() == [1.0, 0.0, 0.0, 0.0]
+    assert ids[2].tolist() == [5, 33, 0, 1]
+
+
+@pytest.mark.parametrize("T,k,E,base", [(77, 8, 66, 0), (128, 8, 66, 0), (129, 31, 256, 100), (511, 8, 256, 0), (1, 1, 1, 0)])
+def test_sort_by_matching(nat, T, k, E, base):
+    ids = torch.randint(0, E + base, (T, k), device=DEV, dtype=torch.int32)
+    ids[::3] = ids[0, 0].clone()                                              # long runs of one expert
+    wts = torch.rand(T, k, device=DEV)
+    rows = torch.full((T * k,), -7.0, device=DEV)
+    seg, src, dest = nat.moe_permute(ids, base, E, wts, rows)
+    order = check_sort(ids, base, E, seg, src, dest)
+    assert torch.equal(rows[:len(order)].cpu(), wts.flatten().cpu()[order])
