@@ -647,7 +647,7 @@ __device__ __forceinline__ void cp16(uint32_t dst, const void * src, bool valid)
 
 template <int NV, int ST>                                    // columns of V per 16: V <= 16 NV; tiles in shared memory
 __global__ void __launch_bounds__(NT) gqa_mma_kernel(const __grid_constant__ jib_gqa a, const bf16 * __restrict__ q, const bf16 * __restrict__ gate,
-                                                     long long ld_gate, bf16 * __restrict__ out, long long ldo, int run, int heads) {
+                                                     long long ld_gate, bf16 * __restrict__ out, long long ldo, int run, int heads, int warm) {
     extern __shared__ __align__(16) uint8_t smem_mma[];
     __shared__ float m_s[ROWS], l_s[ROWS], wm[4][ROWS], wl[4][ROWS];
     PDL_TRIGGER_TOP();
@@ -655,11 +655,24 @@ __global__ void __launch_bounds__(NT) gqa_mma_kernel(const __grid_constant__ jib
     const int LD = D + PADC, LV = V + PADC;                  // row strides (elements)
     const uint32_t q_addr = (uint32_t) __cvta_generic_to_shared(smem_mma), kv_addr = q_addr + ROWS * LD * 2;
     const uint32_t tile_bytes = MK * (LD + LV) * 2;
-    pdl_wait();      // inputs come from earlier kernels; nothing is written before this point
     Work w;
-    if (!find_work(a, run, heads, MK, w)) return;
+    const bool work = find_work(a, run, heads, MK, w);       // from the step's own inputs, which no kernel of the step writes
+    if (!work) {
+        pdl_wait();
+        return;
+    }
+    w.k_hi = max(w.k_hi, w.k_lo);                            // no tiles for this CTA of the cluster: the loop still has its round 0
     const int * bt = a.block_tables + (size_t) w.b * a.max_blocks;
     const bf16 * cache = (const bf16 *) a.cache;
+    if (warm && w.k_lo >= w.pt && w.k_lo < w.k_hi) {
+        // this warp's keys and values of the first tile out of memory into L2 (the step's weights pushed them out); what the step still
+        // writes to them arrives there as well
+        const int p = (w.k_lo + w.t0) * MK + warp * 16 + (lane & 15);
+        if (p >= w.lo && p < w.end) {
+            const bf16 * src = cache + ((size_t) bt[p / a.block_size] * a.block_size + p % a.block_size) * a.row + (lane < 16 ? w.g * D : a.G * D + w.g * V);
+            for (int c = 0; c < (lane < 16 ? D : V); c += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + c));
+        }
+    }
     const int d8 = D / 8, v8 = V / 8;
     // the warp's 16 keys, as 16-byte units that go round the lanes, row after row (several at a time if they are short).  16 adjacent positions
     // of a cache block follow one another; else lane l knows where key l & 15 is
@@ -704,13 +717,18 @@ __global__ void __launch_bounds__(NT) gqa_mma_kernel(const __grid_constant__ jib
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    for (int i = tid; i < ROWS * d8; i += NT) {
-        const int r = i / d8, c = i % d8;
-        cp16(q_addr + (r * LD + c * 8) * 2, q + (r < w.rows ? ((size_t) (w.q0 + w.i0 + r / w.nh) * a.H + w.h0 + r % w.nh) * D + c * 8 : 0), r < w.rows);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    auto start = [&] {
+        pdl_wait();      // queries and rows of this step come from earlier kernels; nothing is written to global memory before this point
+        for (int i = tid; i < ROWS * d8; i += NT) {
+            const int r = i / d8, c = i % d8;
+            cp16(q_addr + (r * LD + c * 8) * 2, q + (r < w.rows ? ((size_t) (w.q0 + w.i0 + r / w.nh) * a.H + w.h0 + r % w.nh) * D + c * 8 : 0), r < w.rows);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < ST - 1; ++i) stage(w.k_lo + i, i);
+        for (int i = 0; i < ST - 1; ++i) stage(w.k_lo + i, i);
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 1) : "memory");
+        __syncthreads();                                     // the queries are there
+    };
     const int fr = lane >> 2, fc = (lane & 3) * 2;
     // positions, first keys and pooled blocks of this thread's two rows
     int pos[2], first[2], blocks[2];
@@ -728,12 +746,21 @@ __global__ void __launch_bounds__(NT) gqa_mma_kernel(const __grid_constant__ jib
         for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
     constexpr float LOG2E = 1.4426950408889634f;
     const float sc = a.softcap > 0.f ? 2.f * LOG2E * a.scale / a.softcap : a.scale * LOG2E, cap = a.softcap * LOG2E;
-    asm volatile("cp.async.wait_group %0;" ::"n"(ST - 1) : "memory");
-    __syncthreads();                                         // the queries are there
-    for (int kt = w.k_lo; kt < w.k_hi; ++kt) {
-        const int buf = (kt - w.k_lo) % ST;
-        stage(kt + ST - 1, (buf + ST - 1) % ST);
-        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 1) : "memory");
+    // A decode CTA goes round this loop once or twice per launch and finds its code cold: in small batches a dry round over whatever the
+    // buffers hold runs while the previous kernel does.  Its results are dropped.  With the rows prefetched and the warps' outputs added up
+    // in one step instead of four, from the previous kernel's end to this one's inside a decode graph of 4 sequences of 200 to 790 keys:
+    // 14.1 -> 9.5 us (full attention), 14.9 -> 10.2 us (window and pooled rows), 12.8 -> 7.8 us (chunks).
+    for (int kt = w.k_lo - 1; kt < w.k_hi; ++kt) {
+        const bool dry = kt < w.k_lo;
+        if (dry && !warm) {
+            start();
+            continue;
+        }
+        const int buf = dry ? 0 : (kt - w.k_lo) % ST;
+        if (!dry) {
+            stage(kt + ST - 1, (buf + ST - 1) % ST);
+            asm volatile("cp.async.wait_group %0;" ::"n"(ST - 1) : "memory");
+        }
         __syncwarp();
         const uint32_t k_addr = kv_addr + buf * tile_bytes + warp * 16 * LD * 2, v_addr = kv_addr + buf * tile_bytes + (MK * LD + warp * 16 * LV) * 2;
         float s[2][4];
@@ -803,6 +830,16 @@ __global__ void __launch_bounds__(NT) gqa_mma_kernel(const __grid_constant__ jib
             mma(o[n + 1], x, y[2], y[3]);
         }
         __syncwarp();                                        // the buffer is free
+        if (dry) {
+#pragma unroll
+            for (int n = 0; n < 2 * NV; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) { m[e] = -INFINITY; l[e] = 0.f; }
+            __syncthreads();                                 // nobody reads what the copies are about to fill
+            start();
+        }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
@@ -815,31 +852,27 @@ __global__ void __launch_bounds__(NT) gqa_mma_kernel(const __grid_constant__ jib
         }
     }
     __syncthreads();
-    // the four warps' outputs, brought to a common maximum, summed in shared memory one warp after the other
+    // the four warps' outputs, brought to a common maximum, side by side in shared memory (4 x ROWS x V numbers: two tiles hold more), then
+    // summed in the order of the warps
     float * part = (float *) (smem_mma + ROWS * LD * 2);
-    float f[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
         const int r = fr + 8 * e;
         const float mx = fmaxf(fmaxf(wm[0][r], wm[1][r]), fmaxf(wm[2][r], wm[3][r]));
-        f[e] = m[e] == -INFINITY ? 0.f : exp2f(m[e] - mx);
+        const float f = m[e] == -INFINITY ? 0.f : exp2f(m[e] - mx);
+#pragma unroll
+        for (int n = 0; n < 2 * NV; ++n)
+            if (n * 8 < V) *(float2 *) (part + (warp * ROWS + r) * V + n * 8 + fc) = make_float2(o[n][2 * e] * f, o[n][2 * e + 1] * f);
     }
-    for (int k = 0; k < 4; ++k) {
-        if (warp == k) {
+    __syncthreads();
+    for (int i = tid * 4; i < ROWS * V; i += NT * 4) {
+        float4 y = *(const float4 *) (part + i);
 #pragma unroll
-            for (int n = 0; n < 2 * NV; ++n) {
-                if (n * 8 >= V) break;
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    float2 * p = (float2 *) (part + (fr + 8 * e) * V + n * 8 + fc);
-                    float2 y = k == 0 ? make_float2(0.f, 0.f) : *p;
-                    y.x += o[n][2 * e] * f[e];
-                    y.y += o[n][2 * e + 1] * f[e];
-                    *p = y;
-                }
-            }
+        for (int k = 1; k < 4; ++k) {
+            const float4 x = *(const float4 *) (part + k * ROWS * V + i);
+            y.x += x.x; y.y += x.y; y.z += x.z; y.w += x.w;
         }
-        __syncthreads();
+        *(float4 *) (part + i) = y;
     }
     if (tid < ROWS) {
         const float mx = fmaxf(fmaxf(wm[0][tid], wm[1][tid]), fmaxf(wm[2][tid], wm[3][tid]));
@@ -885,14 +918,15 @@ bool mma_ok(const jib_gqa & a, const void * q) {
 template <int NV, int ST>
 int launch_mma_as(const jib_gqa & a, const void * q, const void * gate, long long ld_gate, void * out, long long ldo, int single, int splits,
                   cudaStream_t s) {
-    const int tile = MK * (a.D + a.V + 2 * PADC) * 2, smem = ROWS * (a.D + PADC) * 2 + ST * tile;       // >= the [ROWS][V] partial results
+    const int tile = MK * (a.D + a.V + 2 * PADC) * 2, smem = ROWS * (a.D + PADC) * 2 + ST * tile;
+    static_assert(ST >= 2, "the tiles' memory holds the four warps' outputs at the end");
     constexpr int CAP = 220 * 1024;
     static std::atomic<unsigned char> done[jib::MAX_DEVICES];
     if (smem > CAP || !jib::ensure_dyn_smem(gqa_mma_kernel<NV, ST>, CAP, done)) return JIB_E_ARG;
     const int rep = a.H / a.G, heads = rep < ROWS ? rep : ROWS, run = single ? 0 : ROWS / heads;
     const dim3 grid(single ? a.T : a.T / run + a.n_seqs, a.G * ((rep + heads - 1) / heads), splits);
     const cudaError_t e = jib::launch_pdl_cluster(gqa_mma_kernel<NV, ST>, grid, dim3(NT), (size_t) smem, s, splits, a, (const bf16 *) q, (const bf16 *) gate,
-                                                  ld_gate, (bf16 *) out, ldo, run, heads);
+                                                  ld_gate, (bf16 *) out, ldo, run, heads, single ? jib::warm_for(a.T) : 0);
     if (e != cudaSuccess) { (void) cudaGetLastError(); return JIB_E_LAUNCH; }
     return launched();
 }
