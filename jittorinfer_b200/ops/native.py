@@ -215,7 +215,8 @@ def tensor_from_ptr(ptr: int, shape, dtype: torch.dtype, device) -> torch.Tensor
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # what torch.cuda.current_stream().cuda_stream gives, without the objects: a prompt of a few tokens is some 360 launches from Python
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _ck(rc: int, what: str):

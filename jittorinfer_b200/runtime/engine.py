@@ -614,17 +614,17 @@ class LLMEngine:
             self._poison_freed()
         starts = np.concatenate([[0], np.cumsum(lens)])
         rows = [int(s) + int(p) for s, (_, _, want) in zip(starts, entries) for p in want]
-        rows_dev = torch.tensor(rows, dtype=torch.int32).to(self.device)
+        rows_dev = torch.tensor(rows, dtype=torch.int32).to(self.device) if rows else torch.empty(0, dtype=torch.int32, device=self.device)
         # a graph computes every row's logits (row t is sequence t); an eager step computes the wanted ones
         self.io.h["out_rows"][:n_seqs] = np.arange(n_seqs)
         out, graph = self._dispatch(n_tokens, n_seqs, n_seqs if max_q == 1 else 0, max_q, "logits", out_rows=rows_dev)
         self.stats["tokens_out"] += len(rows)
         if graph and rows:
             out = out.index_select(0, rows_dev.long())
+        if self._status_hosts is not None:          # queued ahead of the logits: one wait for both
+            self._status_hosts[0].copy_(self._status_dev, non_blocking=bool(rows))
         res = out.float().cpu() if rows else torch.empty(0, self.hp.n_vocab)
-        if self._status_hosts is not None:
-            self._status_hosts[0].copy_(self._status_dev)
-            self._check_device_status(self._status_hosts[0])
+        self._check_device_status(self._status_hosts[0] if self._status_hosts is not None else None)
         return res
 
     def end_feed(self, key: object) -> None:
