@@ -603,7 +603,7 @@ def moe_gate(g, w_router, bias, k, n_group, topk_group, scale, norm, sigmoid, n_
         _ck(load().jib_moe_gate_sort(g.data_ptr() if own else None, w_router.data_ptr(), _p(bias), _p(logit_bias), logits.data_ptr(), ids.data_ptr(),
                                      wts.data_ptr(), T, d, E, k, n_group, topk_group, float(scale), int(norm), int(sigmoid), n_shared, int(group_top2),
                                      int(shared_gate), expert_base, E_local, seg.data_ptr(), src.data_ptr(), dest.data_ptr(), row_wts.data_ptr(),
-                                     _stream()), "moe_gate_sort")
+                                     _stream()), "moe_gate")
         ids.sorted_pairs = (expert_base, E_local, ids._version, seg, src, dest)
         wts.sorted_pairs = (ids.data_ptr(), wts._version, row_wts)
         return (ids, wts) + ((g,) if pre_norm is not None else ()) + ((logits[:, E],) if shared_gate else ())
