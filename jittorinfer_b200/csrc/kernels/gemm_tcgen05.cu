@@ -1105,6 +1105,186 @@ TilePlan plan_tiles(int N, int K, int T, bool dual, bool can_persist, int sms) {
     return best;
 }
 
+// ---------------------------------------------------------------------------------------------
+// Products of up to 8 tokens with a matrix that one wave of CTAs holds in flight.  A tcgen05 tile of such a product is a chain of fixed
+// costs (tensor memory, a ring of stages, the accumulator's way back, a cluster's sum: 4.5 to 7 us inside a decode graph for 1 to 8 MB
+// that take 0.2 to 1.3 us to read), so here a warp reads 16 rows straight into the fragments of m16n8k16 products, before the wait for the
+// previous kernel, and only the token rows (8 of them are the n of the product, whatever T is) and one barrier follow it.
+// A lane's 16-byte read holds 8 adjacent elements of a row; the product's 16 places along K are numbered so that they are two of its four
+// pairs, for weights and tokens alike.  KS warps share a row's K, the others take further rows; sums meet in shared memory in warp order.
+// ---------------------------------------------------------------------------------------------
+struct NarrowArgs {
+    const __nv_bfloat16 * x, * w, * w2;
+    long long x_row, x_batch, w_row, w_batch;
+};
+constexpr int NARROW_T = 8, NARROW_NT = 256;
+
+__device__ __forceinline__ uint4 ld_stream(const __nv_bfloat16 * p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void mma_16x8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <int KS, bool DUAL, int FN>
+__global__ void __launch_bounds__(NARROW_NT, DUAL ? 1 : 2) gemm_narrow_kernel(const NarrowArgs m, const GemmArgs args) {
+    JIB_KS(1, 0);
+    PDL_TRIGGER_TOP();
+    constexpr int WARPS = NARROW_NT / 32, ROWS = WARPS / KS * 16, UB = 8, MATS = DUAL ? 2 : 1, OUTS = (ROWS * NARROW_T + NARROW_NT - 1) / NARROW_NT;
+    __shared__ float red[MATS][WARPS][NARROW_T][16];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3, ks = warp % KS, rg = warp / KS, batch = blockIdx.y;
+    const int n0 = blockIdx.x * ROWS, nb = args.K / 32, kb0 = nb * ks / KS, kb1 = nb * (ks + 1) / KS;
+    const __nv_bfloat16 * wr[MATS][2];
+#pragma unroll
+    for (int i = 0; i < MATS; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)            // rows past the last one are read as the last one and dropped
+            wr[i][h] = (i == 0 ? m.w : m.w2) + batch * m.w_batch + (long long) min(n0 + rg * 16 + h * 8 + g, args.N - 1) * m.w_row + c * 8;
+    uint4 w[MATS][2][UB];
+#pragma unroll
+    for (int u = 0; u < UB; ++u)
+        if (kb0 + u < kb1)
+#pragma unroll
+            for (int i = 0; i < MATS; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) w[i][h][u] = ld_stream(wr[i][h] + (kb0 + u) * 32);
+    pdl_wait();      // the weights above are launch-invariant; everything else belongs to the stream order
+    JIB_KS(1, 1);
+    const __nv_bfloat16 * xr = m.x + batch * m.x_batch + (long long) min(g, args.T - 1) * m.x_row + c * 8;
+    const bool on = g < args.T;
+    uint4 x[UB];
+#pragma unroll
+    for (int u = 0; u < UB; ++u) x[u] = on && kb0 + u < kb1 ? *(const uint4 *) (xr + (kb0 + u) * 32) : make_uint4(0, 0, 0, 0);
+    // residual and bias of the results this thread will store: requested now
+    float res[OUTS];
+#pragma unroll
+    for (int o = 0; o < OUTS; ++o) {
+        const int i = threadIdx.x + o * NARROW_NT, t = i / ROWS, n = n0 + i % ROWS;
+        res[o] = 0.f;
+        if (t < args.T && n < args.N) {
+            if (FN == 3) res[o] = args.bias[n];
+            else if (args.residual != nullptr) {
+                const long long ri = (long long) batch * args.res_batch_stride + t * args.ldr + n;
+                res[o] = args.res_f32 ? ((const float *) args.residual)[ri] : __bfloat162float(((const __nv_bfloat16 *) args.residual)[ri]);
+            }
+        }
+    }
+    float acc[MATS][2][4];
+#pragma unroll
+    for (int i = 0; i < MATS; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][h][j] = 0.f;
+    for (int kb = kb0; kb < kb1; kb += UB) {
+#pragma unroll
+        for (int u = 0; u < UB; ++u) {
+            if (kb + u < kb1) {
+#pragma unroll
+                for (int i = 0; i < MATS; ++i) {
+                    const uint4 lo = w[i][0][u], hi = w[i][1][u];
+                    mma_16x8(acc[i][0], lo.x, hi.x, lo.y, hi.y, x[u].x, x[u].y);
+                    mma_16x8(acc[i][1], lo.z, hi.z, lo.w, hi.w, x[u].z, x[u].w);
+                }
+                if (kb + UB + u < kb1) {       // the places are free: the next round's elements
+#pragma unroll
+                    for (int i = 0; i < MATS; ++i)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) w[i][h][u] = ld_stream(wr[i][h] + (kb + UB + u) * 32);
+                    if (on) x[u] = *(const uint4 *) (xr + (kb + UB + u) * 32);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < MATS; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) red[i][warp][c * 2 + (j & 1)][g + (j >> 1) * 8] = acc[i][0][j] + acc[i][1][j];
+    __syncthreads();
+#pragma unroll
+    for (int o = 0; o < OUTS; ++o) {
+        const int i = threadIdx.x + o * NARROW_NT, t = i / ROWS, r = i % ROWS, n = n0 + r;
+        if (t >= args.T || n >= args.N) continue;
+        float v[MATS];
+#pragma unroll
+        for (int q = 0; q < MATS; ++q) {
+            v[q] = red[q][r / 16 * KS][t][r & 15];
+#pragma unroll
+            for (int k = 1; k < KS; ++k) v[q] += red[q][r / 16 * KS + k][t][r & 15];
+        }
+        const float f = DUAL ? gated(v[0], args.act) * v[MATS - 1] : function_of<FN>(v[0], args, FN == 2 ? row_factor(args, t, true) : res[o]);
+        const float y = FN == 3 ? f : f + res[o];
+        const long long oi = (long long) batch * args.out_batch_stride + t * args.ldo + n;
+        if (args.out_f32) ((float *) args.out)[oi] = y;
+        else ((__nv_bfloat16 *) args.out)[oi] = __float2bfloat16(y);
+    }
+    JIB_KS(1, 9);
+}
+
+template <int KS, bool DUAL>
+int launch_narrow_as(const NarrowArgs & m, const GemmArgs & a, int batch, cudaStream_t stream) {
+    constexpr int ROWS = NARROW_NT / 32 / KS * 16;
+    const dim3 grid((a.N + ROWS - 1) / ROWS, batch);
+    if (DUAL) JIB_LAUNCH((gemm_narrow_kernel<KS, DUAL, 0>), grid, NARROW_NT, 0, stream, m, a);
+    else if (a.bias != nullptr) JIB_LAUNCH((gemm_narrow_kernel<KS, DUAL, DUAL ? 0 : 3>), grid, NARROW_NT, 0, stream, m, a);
+    else if (a.unary == JIB_UNARY_GELU) JIB_LAUNCH((gemm_narrow_kernel<KS, DUAL, DUAL ? 0 : 2>), grid, NARROW_NT, 0, stream, m, a);
+    else if (a.unary != JIB_UNARY_NONE) JIB_LAUNCH((gemm_narrow_kernel<KS, DUAL, DUAL ? 0 : 1>), grid, NARROW_NT, 0, stream, m, a);
+    else JIB_LAUNCH((gemm_narrow_kernel<KS, DUAL, 0>), grid, NARROW_NT, 0, stream, m, a);
+    return cudaGetLastError() == cudaSuccess ? 0 : JIB_E_LAUNCH;
+}
+
+// Warps that share a row's K: runs of at most 256 elements (a lane's registers), and enough CTAs for the SMs while runs keep 64.
+int narrow_ks(int N, int K, int batch, int sms) {
+    int ks = 1;
+    while (ks < 8 && K / (2 * ks) >= 64 && (K / ks > 256 || (long long) ((N + 128 / ks - 1) / (128 / ks)) * batch < sms)) ks *= 2;
+    return ks;
+}
+
+// Where it is the faster of the two (us on a B200, weights from memory; N x K x heads, 1 / 8 tokens, tcgen05 tiles -> this): 128 x 512 x 16
+// 4.0 / 4.1 -> 2.5 / 2.7; 512 x 128 x 128 7.0 / 7.1 -> 5.2 / 5.8; 2048 x 512 4.0 / 4.1 -> 2.5 / 2.7; 4096 x 1024 4.2 / 4.5 -> 3.6 / 3.9; gated
+// pairs 512 x 512 8.3 / 7.6 -> 1.6 / 1.7, 1408 x 2048 5.4 / 5.8 -> 3.0 / 3.3, 5632 x 2048 15.1 / 16.5 -> 10.2 / 10.7.  Not where a row's run
+// is longer than the 256 elements a lane holds: rounds keep too little in flight (2112 x 5120 6.5 / 6.9 against 11.0 / 11.4), nor at that length
+// (2048 x 2048 4.3 / 4.5 against 4.4 / 4.9, and 3 us slower inside a decode graph); nor for matrices of several waves (128 x 512 x 128
+// 4.8 against 5.1 / 5.6, 32768 x 256 4.5 / 4.7 against 4.7 / 5.4, gated 8192 x 1536 10.0 / 11.2 against 11.7 / 12.1).
+// Whole passes: one conversation 74.8 -> 70.5 ms, four users of lugovik-lite 22.1 -> 21.4 ms.
+bool narrow_size(long long N, long long K, long long batch, bool dual) {
+    const long long mb = (N * K * batch * (dual ? 4 : 2)) >> 20;
+    if (dual) return K <= 2048 && mb < 47;
+    return K <= 128 ? mb <= 32 : K <= 1024 && mb < 12;
+}
+
+bool narrow_ok(const jib_gemm_desc * d, bool dual, int batch) {
+    auto aligned = [](const void * p) { return ((uintptr_t) p & 15) == 0; };
+    return d->T <= NARROW_T && d->seg == nullptr && d->bn == 0 && d->splits <= 0 && d->ar == nullptr && d->ag_flags == nullptr && d->out_row_ptr == nullptr &&
+           d->src_token == nullptr && d->K % 32 == 0 && d->x_row_stride % 8 == 0 && d->w_row_stride % 8 == 0 &&
+           (batch == 1 || (d->x_batch_stride % 8 == 0 && d->w_batch_stride % 8 == 0)) && aligned(d->x) && aligned(d->w) && (!dual || aligned(d->w2)) &&
+           batch <= 65535 && narrow_size(d->N, d->K, batch, dual);
+}
+
+int launch_narrow(const jib_gemm_desc * d, bool dual, int batch, cudaStream_t stream) {
+    GemmArgs a;
+    memset(&a, 0, sizeof(a));
+    a.out = d->out; a.residual = d->residual; a.ldo = d->ldo; a.out_batch_stride = d->out_batch_stride; a.ldr = d->ldr;
+    a.res_batch_stride = d->res_batch_stride; a.T = d->T; a.N = d->N; a.K = d->K; a.out_f32 = d->out_f32; a.res_f32 = d->res_f32;
+    a.act = d->act; a.unary = dual ? JIB_UNARY_NONE : d->unary; a.scale = d->scale; a.softcap = d->softcap; a.row_scale = d->row_scale;
+    a.cap2 = d->softcap > 0.f ? 2.f * d->scale / d->softcap : 0.f;
+    if (d->residual != nullptr && d->ldr == 0 && d->res_f32 && !dual && batch == 1 && a.unary == JIB_UNARY_NONE) {
+        a.bias = (const float *) d->residual;
+        a.residual = nullptr;
+    }
+    const NarrowArgs m = {(const __nv_bfloat16 *) d->x, (const __nv_bfloat16 *) d->w, (const __nv_bfloat16 *) d->w2, d->x_row_stride, d->x_batch_stride,
+                          d->w_row_stride, d->w_batch_stride};
+    switch (narrow_ks(d->N, d->K, batch, d->sm_count > 0 ? d->sm_count : 148)) {
+        case 1: return dual ? launch_narrow_as<1, true>(m, a, batch, stream) : launch_narrow_as<1, false>(m, a, batch, stream);
+        case 2: return dual ? launch_narrow_as<2, true>(m, a, batch, stream) : launch_narrow_as<2, false>(m, a, batch, stream);
+        case 4: return dual ? launch_narrow_as<4, true>(m, a, batch, stream) : launch_narrow_as<4, false>(m, a, batch, stream);
+        default: return dual ? launch_narrow_as<8, true>(m, a, batch, stream) : launch_narrow_as<8, false>(m, a, batch, stream);
+    }
+}
+
 template <int BN, bool DUAL, int FN>
 int launch_as(const CUtensorMap & a, const CUtensorMap & a2, const CUtensorMap & b, const GemmArgs & args, dim3 grid,
            cudaStream_t stream) {
@@ -1169,6 +1349,7 @@ extern "C" JIB_EXPORT int jib_gemm_bf16(const jib_gemm_desc * d, void * stream_)
     const bool src_mode = d->src_token != nullptr;
     if (src_mode && (!grouped || d->src_rows <= 0 || d->src_rows > 256 || d->ar != nullptr)) return JIB_E_ARG;
     const int rows_bound = src_mode ? d->src_rows : grouped ? (d->max_rows > 0 ? d->max_rows : d->T) : d->T;
+    if (narrow_ok(d, dual, batch)) return launch_narrow(d, dual, batch, stream);
     int bn = d->bn;
     if (bn == 0) {
         bn = 16;
