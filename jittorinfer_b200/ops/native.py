@@ -41,6 +41,8 @@ EXPERT_LIST = os.environ.get("JIB_EXPERT_LIST", "1") == "1"
 # Grouped launches of prompt chunks walk a list of the (expert, token tile) pairs that exist.
 TILE_LIST = os.environ.get("JIB_TILE_LIST", "1") == "1"
 TILE_LIST_MIN_PAIRS = 1024
+# Grouped launches of few rows per expert in tiles of 16 rows: for this many tokens; idle CTAs past which they walk a list.
+SMALL_TILES_MIN_T, SMALL_TILES_MAX_T, SMALL_TILES_MAX_IDLE = 24, 80, 20000
 # The router launch of a decode batch also applies the RMSNorm of its input ("0": a separate norm launch before it).
 ROUTE_NORM = os.environ.get("JIB_ROUTE_NORM", "1") == "1"
 FUSED_ROUTE_MAX_T = 16                      # past this the separate router's tiles add up in another order (and are faster)
@@ -714,6 +716,16 @@ def moe_routed(x, ids, wts, wg, wu, wd, expert_base=0, n_expert=None):
     active = min(E_local, T * k)
     if ACTIVE_HINT_EXPECTED and n_expert:        # split-K sized for the experts a batch is expected to hit, not for all
         active = min(active, expected_active_experts(T, k, E_local, n_expert))
+    if SMALL_TILES_MIN_T <= T <= SMALL_TILES_MAX_T and T * k <= 10 * E_local:
+        # A dozen pairs an expert at most, nearly all experts hit: what counts is the stream of weights, and it runs best past tiles of 16
+        # rows, two CTAs on an SM (64 tokens x 8 over 64 + 2 experts of 3 x 1408 x 2048: 208.7 us with every expert multiplying all 64 tokens,
+        # 177.7 so, 177 at the rate of a copy; 32 tokens 186 -> 170, 77 tokens 190 -> 178; 160 + 2 experts of 3 x 1536 x 5120: 32 tokens 835 ->
+        # 776, 64 tokens 1088 -> 1011).  Below 24 tokens the rows in place are as fast, past 80 tiles of 128 rows.  The grid has a
+        # CTA for every tile that an expert could have; from some 20000 idle ones on (70 us at 25000) a list of the tiles is cheaper (6 us).
+        idle = E_local * ((T + 15) // 16 - 1) * ((wg.shape[1] + 127) // 128 + (wd.shape[1] + 127) // 128)
+        tl = moe_tile_list(seg, E_local, 16, T * k) if idle > SMALL_TILES_MAX_IDLE else None
+        h = gemm_grouped(gather_rows(x, src), seg, wg, wu, T, active, pdl_flags=pair[0], n_slots=slots, bn=16, tile_list=tl, gelu_scale=fn)
+        return gemm_grouped(h, seg, wd, None, T, active, pdl_flags=pair[1], n_slots=slots, bn=16, tile_list=tl), dest
     if TILE_LIST and T * k >= TILE_LIST_MIN_PAIRS:
         # prompt chunks: an expert holds ~T*k/E rows, far fewer than the T the grid would have to be sized for; both grouped
         # launches walk a device-built list of the (expert, 128-token tile) pairs that exist
