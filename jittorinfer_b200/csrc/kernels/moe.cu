@@ -154,169 +154,243 @@ __global__ void __launch_bounds__(GATE_NT) router_logits_kernel(const bf16 * __r
     JIB_KS(9, 9);
 }
 
-// The same logits for batches of more than ROUTER_ROWS_MAX tokens, as tiles.  router_logits_kernel reads its expert's tokens once per 8
-// of them and converts every element for one multiplication; what bounds this kernel is shared-memory reads beside the fp32 pipe.
-// A CTA owns RT_T tokens x RT_E experts over one of gridDim.z runs of the d axis; its 8 warps take 8 of every 64 elements each (a lane: 4
-// tokens x 8 experts, packed fp32 pairs along d, so that one 16-byte read feeds eight multiplications), add up through shared memory, and
-// the CTAs of a cluster through distributed shared memory in rank order: no sum depends on timing.  Tiles of 16 tokens rather than 32:
-// 64 tokens have only 4 tiles; at 2048 tokens 8 x 8 per lane with one CTA per SM measured 32.6 against 34.1 us, at 777 (d 5120) 120 against 74.
-// Router rows of the first stages are requested before the wait for the previous kernel.
-// Router and gate on a B200, before -> now (us): 64 experts x 2048: 32 tokens 11.8 -> 10.7, 64 17.1 -> 10.7, 333 35.2 -> 13.9, 2048 101 -> 34;
-// 160 x 5120: 17 tokens 22.8 -> 18.9, 64 54.7 -> 18.4, 2048 489 -> 198.  2-norm error against 64 bits 0.99e-7 -> 1.04 .. 1.1e-7 (one
-// rounding of the result is 0.6e-7).
-constexpr int RT_T = 16, RT_E = 64, RT_K = 64, RT_STAGES = 3, RT_NT = 256;
+// The same logits, bit for bit, for batches of more than ROUTER_ROWS_MAX tokens, as tiles.  router_logits_kernel reads its expert's tokens
+// once per 8 of them and converts every element for one multiplication; what bounds this kernel is shared-memory reads beside the fp32 pipe.
+// A CTA owns RT_T tokens x RT_E experts.  The order of the sums is that of router_rows, so that a token's logits do not depend on how many
+// tokens are beside it: 2048 elements are 8 spans (the warps there) of 32 vectors (its lanes), a vector is a chain of 8 multiplications, the
+// vectors 2048 apart are added up, then vectors of a span pairwise 16, 8, 4, 2 and 1 apart, then the spans in order.  Here a chunk is 64
+// adjacent elements, warp g takes vector g of each (a lane: 4 tokens x 4 experts); the chunks of a span come in the order 0, 2, 1, 3 (vectors
+// g, g + 16, g + 8, g + 24: their sums are the first two levels), and the 8 warps' sums of a span meet in shared memory (the other three).
+// gridDim.z CTAs of a cluster take runs of spans; rank 0 adds their sums up in order.
+// Tiles of 16 tokens x 32 experts with three CTAs on an SM: 64 tokens x 64 experts are 8 tiles, and the chains of multiplications in front of every
+// addition need the warps (16 x 64, two CTAs: 16.5 against 10.7 us at 64 tokens, 44.0 against 41.3 at 2048).  Four stages: the same.  Router rows
+// of the first stages are requested before the wait for the previous kernel.
+// Router and gate on a B200, row kernel -> this (us): 64 experts x 2048: 17 tokens 10.4 -> 9.2, 64 17.1 -> 10.7, 333 35.0 -> 14.1, 2048 100 -> 41.3;
+// 160 x 5120: 17 tokens 22.1 -> 21.1, 64 56.8 -> 23.1, 2048 557 -> 193.  2-norm error against 64 bits as there: 0.99e-7 and 1.05e-7.  Sums in any
+// order that keeps packed pairs along d instead: 64 x 2048 9.9 us at 64 tokens, 32.8 at 2048, but errors of 1.04e-7 to 1.36e-7.
+constexpr int RT_T = 16, RT_E = 32, RT_J = RT_E / 8, RT_K = 64, RT_STAGES = 3, RT_NT = 256;
+constexpr int RT_SPAN = 256, RT_SPANS = 8, RT_TURN = RT_SPAN * RT_SPANS;     // elements of a span, spans, and what they cover together
 constexpr int RT_WROW = RT_K * 4 + 16, RT_GROW = RT_K * 2 + 16;            // padded rows: 8 experts (4 tokens) of a warp's read meet no bank twice
 constexpr int RT_STAGE = RT_E * RT_WROW + RT_T * RT_GROW;
-constexpr int RT_FLUSH = 4;                                                  // chunks a register sum runs over
-constexpr int RT_SMEM = RT_STAGES * RT_STAGE + (RT_NT / 32) * RT_T * RT_E * 4;
+constexpr int RT_OUT = RT_T * RT_E, RT_PER = RT_OUT / RT_NT;
+constexpr int RT_SMEM = RT_STAGES * RT_STAGE + (RT_NT / 32) * RT_OUT * 4 + RT_SPANS / 2 * RT_OUT * 4;
 
 __device__ __forceinline__ void cp16_or_zero(uint32_t dst, const void * src, bool on) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
 }
-__device__ __forceinline__ void fma2(float2 & c, float2 a, float2 b) {
-    unsigned long long & x = reinterpret_cast<unsigned long long &>(c);
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(x) : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)));
-}
 
-__global__ void __launch_bounds__(RT_NT, 2) router_tile_kernel(const bf16 * __restrict__ g, const float * __restrict__ w_router,
+// The chunks of spans [s0, s1) in the order of the sums: span, quarter (0, 2, 1, 3), turn.
+struct RouterChunks {
+    int d, span, q, turn;
+    __device__ __forceinline__ int col() const { return turn * RT_TURN + span * RT_SPAN + ((q & 1) * 2 + (q >> 1)) * RT_K; }
+    __device__ __forceinline__ int turns() const { return (d - span * RT_SPAN + RT_TURN - 1) / RT_TURN; }
+    __device__ __forceinline__ void next() {
+        if (++turn == turns()) {
+            turn = 0;
+            if (++q == 4) { q = 0; ++span; }
+        }
+    }
+};
+
+template <bool ONE>      // one turn: d <= RT_TURN
+__global__ void __launch_bounds__(RT_NT, 3) router_tile_kernel(const bf16 * __restrict__ g, const float * __restrict__ w_router,
                                                                float * __restrict__ logits, int T, int d, int E) {
     PDL_TRIGGER_TOP();
     extern __shared__ __align__(16) uint8_t rt_smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int e0 = blockIdx.x * RT_E, t0 = blockIdx.y * RT_T, S = gridDim.z;
-    const int n_chunks = (d + RT_K - 1) / RT_K;
-    const int c0 = (int) ((long long) n_chunks * blockIdx.z / S), c1 = (int) ((long long) n_chunks * (blockIdx.z + 1) / S);
+    const int n_spans = min((d + RT_SPAN - 1) / RT_SPAN, RT_SPANS);
+    const int s0 = n_spans * (int) blockIdx.z / S, s1 = n_spans * ((int) blockIdx.z + 1) / S;
     const uint32_t base = (uint32_t) __cvta_generic_to_shared(rt_smem);
     float * part = (float *) (rt_smem + RT_STAGES * RT_STAGE);             // [warp][token][expert ^ 8 (token mod 4)]
-    auto load_w = [&](int c) {                 // rows past E and columns past d are zeros
-        const uint32_t dst = base + (c - c0) % RT_STAGES * RT_STAGE;
+    float * spans = part + (RT_NT / 32) * RT_OUT;                          // [span of this rank][token][expert]: ranks past 0
+    auto load_w = [&](int stage, int col) {      // rows past E and columns past d are zeros
+        const uint32_t dst = base + stage * RT_STAGE;
 #pragma unroll
         for (int i = tid; i < RT_E * (RT_K / 4); i += RT_NT) {
             const int e = i / (RT_K / 4), k = i % (RT_K / 4) * 4;
-            const bool on = e0 + e < E && c * RT_K + k < d;
-            cp16_or_zero(dst + e * RT_WROW + k * 4, on ? w_router + (size_t) (e0 + e) * d + c * RT_K + k : w_router, on);
+            const bool on = e0 + e < E && col + k < d;
+            cp16_or_zero(dst + e * RT_WROW + k * 4, on ? w_router + (size_t) (e0 + e) * d + col + k : w_router, on);
         }
     };
-    auto load_g = [&](int c) {
-        const uint32_t dst = base + (c - c0) % RT_STAGES * RT_STAGE + RT_E * RT_WROW;
+    auto load_g = [&](int stage, int col) {
+        const uint32_t dst = base + stage * RT_STAGE + RT_E * RT_WROW;
         if (tid < RT_T * (RT_K / 8)) {
             const int t = tid / (RT_K / 8), k = tid % (RT_K / 8) * 8;
-            const bool on = t0 + t < T && c * RT_K + k < d;
-            cp16_or_zero(dst + t * RT_GROW + k * 2, on ? g + (size_t) (t0 + t) * d + c * RT_K + k : g, on);
+            const bool on = t0 + t < T && col + k < d;
+            cp16_or_zero(dst + t * RT_GROW + k * 2, on ? g + (size_t) (t0 + t) * d + col + k : g, on);
         }
     };
+    RouterChunks ahead = {d, s0, 0, 0};
+    int filled = 0;      // the stage that is filled next; used: the one that is read next
+    {
+        RouterChunks c = ahead;
 #pragma unroll
-    for (int s = 0; s < RT_STAGES - 1; ++s)
-        if (c0 + s < c1) load_w(c0 + s);
+        for (int s = 0; s < RT_STAGES - 1; ++s)
+            if (c.span < s1) { load_w(s, c.col()); c.next(); }
+    }
     pdl_wait();      // inputs come from earlier kernels; nothing is written before this point
 #pragma unroll
     for (int s = 0; s < RT_STAGES - 1; ++s) {
-        if (c0 + s < c1) load_g(c0 + s);
+        if (ahead.span < s1) { load_g(s, ahead.col()); ahead.next(); }
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
+    filled = RT_STAGES - 1;
+    int used = 0;
     const int eg = lane & 7, tg = lane >> 3;      // experts eg + 8 j, tokens tg + 4 i
-    float2 acc[4][8];
+    float sum[RT_PER];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int r = 0; r < RT_PER; ++r) sum[r] = 0.f;
+    // the warps' sums of a span, vectors 4, 2 and 1 apart
+    auto meet = [&](int span) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
-    // A sum over d / 16 terms in a row would lose up to three times as much to rounding as sums of 16 that are added up
-    // (5120 elements: 3.3e-7 against 1.1e-7): every few chunks the registers are added to this thread's places in shared memory.
-    bool first = true;
-    auto flush = [&] {
+        for (int r = 0; r < RT_PER; ++r) {
+            const int o = tid + r * RT_NT;
+            float v[RT_NT / 32];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float & p = part[(warp * RT_T + tg + 4 * i) * RT_E + ((eg + 8 * j) ^ (8 * tg))];
-                p = (first ? 0.f : p) + (acc[i][j].x + acc[i][j].y);
-                acc[i][j] = make_float2(0.f, 0.f);
-            }
-        first = false;
+            for (int q = 0; q < RT_NT / 32; ++q) v[q] = part[q * RT_OUT + (o ^ (o / RT_E % 4 * 8))];
+            const float s = ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
+            sum[r] += s;
+            if (S > 1) spans[(span - s0) * RT_OUT + o] = s;
+        }
     };
-    for (int c = c0; c < c1; ++c) {
-        if (c > c0 && (c - c0) % RT_FLUSH == 0) flush();
+    // acc += this warp's vector of the next chunk
+    auto take = [&](float (&acc)[4][RT_J], int meet_span) {
         asm volatile("cp.async.wait_group %0;" ::"n"(RT_STAGES - 2) : "memory");
-        __syncthreads();      // chunk c is here for everybody, and nobody reads the stage that is filled next
-        if (c + RT_STAGES - 1 < c1) { load_w(c + RT_STAGES - 1); load_g(c + RT_STAGES - 1); }
+        __syncthreads();      // the chunk is here for everybody, nobody reads the stage that is filled next, and all sums of meet_span are there
+        if (meet_span >= s0) meet(meet_span);
+        if (ahead.span < s1) {
+            load_w(filled, ahead.col());
+            load_g(filled, ahead.col());
+            ahead.next();
+        }
+        filled = filled + 1 == RT_STAGES ? 0 : filled + 1;
         asm volatile("cp.async.commit_group;" ::: "memory");
-        const uint8_t * st = rt_smem + (c - c0) % RT_STAGES * RT_STAGE;
+        const uint8_t * st = rt_smem + used * RT_STAGE + warp * 32;
+        used = used + 1 == RT_STAGES ? 0 : used + 1;
+        float x[4][8];
 #pragma unroll
-        for (int h = 0; h < RT_K / 32; ++h) {
-            const int k = warp * (RT_K / 8) + h * 4;
-            float2 x[4][2];
+        for (int i = 0; i < 4; ++i) {
+            const uint4 v = *(const uint4 *) (st + RT_E * RT_WROW + (tg + 4 * i) * RT_GROW - warp * 16);
+            const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                x[i][2 * k] = __uint_as_float(u[k] << 16);
+                x[i][2 * k + 1] = __uint_as_float(u[k] & 0xffff0000u);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < RT_J; ++j) {
+            const float4 a = *(const float4 *) (st + (eg + 8 * j) * RT_WROW), b = *(const float4 *) (st + (eg + 8 * j) * RT_WROW + 16);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const uint2 v = *(const uint2 *) (st + RT_E * RT_WROW + (tg + 4 * i) * RT_GROW + k * 2);
-                x[i][0] = make_float2(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u));
-                x[i][1] = make_float2(__uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float4 w = *(const float4 *) (st + (eg + 8 * j) * RT_WROW + k * 4);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    fma2(acc[i][j], x[i][0], make_float2(w.x, w.y));
-                    fma2(acc[i][j], x[i][1], make_float2(w.z, w.w));
-                }
+                // as the compiler contracts router_rows' sum of products
+                float p = __fmaf_rn(a.x, x[i][0], __fmul_rn(a.y, x[i][1]));
+                p = __fmaf_rn(a.z, x[i][2], p);
+                p = __fmaf_rn(a.w, x[i][3], p);
+                p = __fmaf_rn(b.x, x[i][4], p);
+                p = __fmaf_rn(b.y, x[i][5], p);
+                p = __fmaf_rn(b.z, x[i][6], p);
+                p = __fmaf_rn(b.w, x[i][7], p);
+                acc[i][j] = __fadd_rn(acc[i][j], p);
             }
         }
-    }
-    flush();
-    __syncthreads();
-    float sum[RT_T * RT_E / RT_NT];
+    };
+    for (int span = s0; span < s1; ++span) {
+        const int turns = RouterChunks{d, span, 0, 0}.turns();
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+            float v[4][RT_J];
 #pragma unroll
-    for (int r = 0; r < RT_T * RT_E / RT_NT; ++r) {
-        const int o = tid + r * RT_NT;
-        float v[RT_NT / 32];
+            for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int q = 0; q < RT_NT / 32; ++q) v[q] = part[q * RT_T * RT_E + (o ^ (o / RT_E % 4 * 8))];
-        sum[r] = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
-    }
-    if (S > 1) {      // the CTAs of the cluster are the runs of d: rank 0 adds them up
-        __syncthreads();
+                for (int j = 0; j < RT_J; ++j) v[i][j] = 0.f;
+            if (ONE) {
+#pragma unroll 1
+                for (int n = 0; n < 2; ++n) take(v, half == 0 && n == 0 ? span - 1 : -1);
+            } else {
+                float y[4][RT_J];
 #pragma unroll
-        for (int r = 0; r < RT_T * RT_E / RT_NT; ++r) part[tid + r * RT_NT] = sum[r];
-        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        if (blockIdx.z == 0) {
-            for (int z = 1; z < S; ++z)
+                for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int r = 0; r < RT_T * RT_E / RT_NT; ++r) {
-                    uint32_t remote;
-                    float v;
-                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(base + RT_STAGES * RT_STAGE + (uint32_t) (tid + r * RT_NT) * 4), "r"(z));
-                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
-                    sum[r] += v;
+                    for (int j = 0; j < RT_J; ++j) y[i][j] = 0.f;
+#pragma unroll 1
+                for (int n = 0; n < turns; ++n) take(v, half == 0 && n == 0 ? span - 1 : -1);
+#pragma unroll 1
+                for (int n = 0; n < turns; ++n) take(y, -1);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < RT_J; ++j) v[i][j] = __fadd_rn(v[i][j], y[i][j]);
+            }
+            // the halves' sums in this thread's places; those of the span before were read two barriers ago at least
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < RT_J; ++j) {
+                    float & p = part[(warp * RT_T + tg + 4 * i) * RT_E + ((eg + 8 * j) ^ (8 * tg))];
+                    p = half == 0 ? v[i][j] : __fadd_rn(p, v[i][j]);
                 }
+        }
+    }
+    __syncthreads();
+    if (s1 > s0) meet(s1 - 1);
+    if (S > 1) {      // each rank adds up a share of the results
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const int share = RT_OUT / S;
+        if (tid < share) {
+            const int o = blockIdx.z * share + tid, t = t0 + o / RT_E, e = e0 + o % RT_E;
+            const uint32_t at = (uint32_t) __cvta_generic_to_shared(spans + o);
+            float v[RT_SPANS], all = 0.f;
+            int z = 0;
+#pragma unroll
+            for (int s = 0; s < RT_SPANS; ++s) {
+                v[s] = 0.f;
+                if (s < n_spans) {
+                    if (s == n_spans * (z + 1) / S) ++z;      // the rank that holds span s
+                    uint32_t remote;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at + (s - n_spans * z / S) * RT_OUT * 4), "r"(z));
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[s]) : "r"(remote) : "memory");
+                }
+            }
+#pragma unroll
+            for (int s = 0; s < RT_SPANS; ++s) all += v[s];
+            if (t < T && e < E) logits[(size_t) t * E + e] = all;
         }
         asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");      // shared memory stays until it was read
-        if (blockIdx.z != 0) return;
+        return;
     }
 #pragma unroll
-    for (int r = 0; r < RT_T * RT_E / RT_NT; ++r) {
+    for (int r = 0; r < RT_PER; ++r) {
         const int o = tid + r * RT_NT, t = t0 + o / RT_E, e = e0 + o % RT_E;
         if (t < T && e < E) logits[(size_t) t * E + e] = sum[r];
     }
 }
 
-// Which of the two: with few tokens the split over experts has more CTAs and shorter chains (64 x 2048, one kernel each: 16 tokens 8.6
-// against 10.4 us, 32 tokens 11.8 against 10.7).
+// Which of the two: with few tokens the split over experts has more CTAs and shorter chains (64 x 2048, with the gate: 16 tokens 8.2 us there,
+// 17 tokens 10.4 there and 9.2 here).
 constexpr int ROUTER_ROWS_MAX = 16;
 
-int launch_router(const bf16 * g, const float * w_router, float * logits, int T, int d, int E, cudaStream_t stream) {
-    if (T <= ROUTER_ROWS_MAX) {
-        JIB_LAUNCH((router_logits_kernel), dim3(E, (T + 63) / 64), GATE_NT, 0, stream, g, w_router, logits, T, d, E, jib::warm_for(T));
-        return cudaGetLastError() == cudaSuccess ? 0 : JIB_E_LAUNCH;
-    }
+template <bool ONE>
+int launch_router_tiles(const bf16 * g, const float * w_router, float * logits, int T, int d, int E, cudaStream_t stream) {
     static std::atomic<unsigned char> attr_done[jib::MAX_DEVICES];
-    if (!jib::ensure_dyn_smem(router_tile_kernel, RT_SMEM, attr_done)) return JIB_E_LAUNCH;
+    const int sms = jib::sm_count();
+    if (sms <= 0 || !jib::ensure_dyn_smem(router_tile_kernel<ONE>, RT_SMEM, attr_done)) return JIB_E_LAUNCH;
     const dim3 tiles((E + RT_E - 1) / RT_E, (T + RT_T - 1) / RT_T);
-    // as many runs of d (up to a portable cluster, at least two chunks each) as two CTAs per SM take at a time
+    // as many runs of spans (up to a portable cluster) as three CTAs per SM take at a time (twice as many: 777 x 64 x 2048 21.9 -> 26.7 us)
     int S = 1;
-    while (S < 8 && (long long) tiles.x * tiles.y * 2 * S <= 2 * 148 && 4 * S <= (d + RT_K - 1) / RT_K) S *= 2;
-    if (jib::launch_pdl_cluster(router_tile_kernel, dim3(tiles.x, tiles.y, S), dim3(RT_NT), RT_SMEM, stream, S, g, w_router, logits, T, d, E) != cudaSuccess)
+    while (S < 8 && (long long) tiles.x * tiles.y * 2 * S <= 3 * sms && 2 * S * RT_SPAN <= d) S *= 2;
+    if (jib::launch_pdl_cluster(router_tile_kernel<ONE>, dim3(tiles.x, tiles.y, S), dim3(RT_NT), RT_SMEM, stream, S, g, w_router, logits, T, d, E) !=
+        cudaSuccess)
         return JIB_E_LAUNCH;
     return 0;
+}
+
+int launch_router(const bf16 * g, const float * w_router, float * logits, int T, int d, int E, cudaStream_t stream) {
+    if (T > ROUTER_ROWS_MAX)
+        return d <= RT_TURN ? launch_router_tiles<true>(g, w_router, logits, T, d, E, stream) : launch_router_tiles<false>(g, w_router, logits, T, d, E, stream);
+    JIB_LAUNCH((router_logits_kernel), dim3(E, (T + 63) / 64), GATE_NT, 0, stream, g, w_router, logits, T, d, E, jib::warm_for(T));
+    return cudaGetLastError() == cudaSuccess ? 0 : JIB_E_LAUNCH;
 }
 
 // Gating of one token by one warp: softmax/sigmoid over the logits, optional group-limited masking, k rounds of arg-max.  A lane holds the

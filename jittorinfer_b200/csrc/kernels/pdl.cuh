@@ -57,6 +57,17 @@ inline bool ensure_dyn_smem(K kern, int bytes, std::atomic<unsigned char> (&done
     return true;
 }
 
+// SMs of the current device (0: no answer).
+inline int sm_count() {
+    static std::atomic<int> known[MAX_DEVICES];
+    int dev = -1, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return 0;
+    if ((n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    known[dev].store(n, std::memory_order_relaxed);
+    return n;
+}
+
 // Small latency-bound kernels run their body twice: once "dry" (same instructions, no stores, indices that come from memory
 // replaced by safe ones) while they still wait for the previous kernel, then for real.  A kernel's first pass over cold code
 // costs an instruction-cache miss every few instructions; the dry pass takes those misses in the shadow of the previous

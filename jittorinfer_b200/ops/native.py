@@ -25,7 +25,7 @@ PERMUTE_MULTI = os.environ.get("JIB_PERMUTE_MULTI", "1") == "1"
 PERMUTE_MULTI_MIN = 4096
 # [RMSNorm +] router logits + gating + expert sort in one launch for decode batches (<= FUSED_ROUTE_MAX_T tokens).  Off by
 # default: measured on B200 the single CTA that gates and sorts after the last logit arrives costs as much as the three
-# launches it replaces (profiles/decode_switches_ab_lite.md).
+# launches it replaces.
 FUSED_ROUTE = os.environ.get("JIB_FUSED_ROUTE", "0") == "1"
 # Grouped-GEMM split-K hint from the expected number of experts hit instead of all local experts.
 ACTIVE_HINT_EXPECTED = os.environ.get("JIB_ACTIVE_HINT", "0") == "1"
@@ -45,7 +45,7 @@ TILE_LIST_MIN_PAIRS = 1024
 SMALL_TILES_MIN_T, SMALL_TILES_MAX_T, SMALL_TILES_MAX_IDLE = 24, 80, 20000
 # The router launch of a decode batch also applies the RMSNorm of its input ("0": a separate norm launch before it).
 ROUTE_NORM = os.environ.get("JIB_ROUTE_NORM", "1") == "1"
-FUSED_ROUTE_MAX_T = 16                      # past this the separate router's tiles add up in another order (and are faster)
+FUSED_ROUTE_MAX_T = 64
 GATE_SORT_MAX_T = 64                        # gate and expert sort as one launch: every token is a warp of one CTA
 _route_stash: Dict[tuple, tuple] = {}       # (ids ptr, expert_base, E_local) -> (seg, src, dest) produced by the fused launch
 

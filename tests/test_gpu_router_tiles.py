@@ -39,6 +39,28 @@ def test_logits(nat, T, E, d, shared_gate):
     assert torch.equal(ids[:, :4].long(), want)
 
 
+def logits_of(nat, x, w):
+    T, d = x.shape
+    E = w.shape[0]
+    logits, ids, wts = torch.empty(T, E, device=DEV), torch.empty(T, 2, dtype=torch.int32, device=DEV), torch.empty(T, 2, device=DEV)
+    nat._ck(nat.load().jib_moe_gate(x.data_ptr(), w.data_ptr(), None, None, logits.data_ptr(), ids.data_ptr(), wts.data_ptr(), T, d, E, 2, 1, 1, 1.0,
+                                    0, 0, 0, 0, 0, nat._stream()), "moe_gate")
+    return logits
+
+
+# spans of 256 elements: one, a part of one, fewer than 8, each number of CTAs of a cluster; turns of 2048: one, a part of the second, all four
+@pytest.mark.parametrize("T", [17, 40, 333, 2500])
+@pytest.mark.parametrize("E,d", [(64, 2048), (7, 8), (65, 264), (130, 776), (160, 5120), (64, 1544), (32, 2056), (66, 8192)])
+def test_a_token_has_the_same_logits_in_any_batch(nat, T, E, d):
+    gen = torch.Generator(device=DEV).manual_seed(T + d)
+    x = torch.randn(T, d, generator=gen, device=DEV).bfloat16()
+    w = torch.randn(E, d, generator=gen, device=DEV) * d ** -0.5
+    w[2, d // 2] = float("inf")
+    some = torch.cat([logits_of(nat, x[t:t + 16].contiguous(), w) for t in range(0, T, 16)])
+    assert bool((x[:, d // 2] != 0).all()) and bool(torch.isinf(some[:, 2]).all())
+    assert torch.equal(logits_of(nat, x, w), some)
+
+
 def test_rows_past_the_last_expert_are_not_read(nat):
     """An infinity in a neighbouring allocation's row must not reach the sums: 65 experts of a matrix of 66 rows, the last one infinite."""
     gen = torch.Generator(device=DEV).manual_seed(5)
