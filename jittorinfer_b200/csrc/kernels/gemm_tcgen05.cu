@@ -1365,9 +1365,11 @@ extern "C" JIB_EXPORT int jib_gemm_bf16(const jib_gemm_desc * d, void * stream_)
     if (d->ar != nullptr && (((const JibArCtx *) d->ar)->d_max % 8 != 0 || d->out_f32)) vec_store = false;
     // One matrix, nobody else's choice, more tokens than one narrow tile: the measured cost model chooses.  Up to 32 tokens the split rules
     // below stand (they are tuned inside decode graphs), and so does the covering tile for matrices of more than two waves of feature tiles
-    // (output heads: every choice streams the weights at the same rate).
+    // (output heads: every choice streams the weights at the same rate).  fp32 results keep that rule as well: the longer a tile's run along
+    // K, the larger the error of the tensor cores' sums (2048 x 2048 at 333 tokens: 4.7e-7 of the result in 4 splits, 2.1e-6 in one), which
+    // a 16-bit result (1.7e-3) does not show.
     const bool planned = d->bn == 0 && d->splits <= 0 && !grouped && batch == 1 && d->ar == nullptr && d->ag_flags == nullptr &&
-                         rows_bound > 32 && n_tiles <= 2 * sms;
+                         !d->out_f32 && rows_bound > 32 && n_tiles <= 2 * sms;
     TilePlan plan = {0, 0};
     if (planned) {
         plan = plan_tiles(d->N, d->K, rows_bound, dual, vec_store && !jib_no_persist(), sms);

@@ -52,3 +52,14 @@ def test_planned_gated_pairs(nat, T):
     lim = 2.0 ** -8 * ref.abs() + 1.1 * d * ((x.double().abs() @ wg.double().abs().T) * b.abs() + (x.double().abs() @ wu.double().abs().T) * (a.abs() + 1))
     assert bool(((nat.gemm(x, wg, wu).double() - ref).abs() <= lim).all())
     nat.check_status()
+
+
+@pytest.mark.parametrize("T,tile", [(33, 64), (100, 128), (333, 256)])
+@pytest.mark.parametrize("N,K", [(2048, 2048), (2112, 5120), (1024, 1024)])
+def test_results_of_32_bits_are_those_of_the_covering_tile(nat, T, tile, N, K):
+    """Fewer splits mean longer sums in the tensor cores: only results that are rounded to 16 bits take the cost model's choice."""
+    g = torch.Generator(device=DEV).manual_seed(T + N)
+    x = torch.randn(T, K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    y = nat.gemm(x, w, out_dtype=torch.float32)
+    assert torch.equal(y, nat.gemm(x, w, out_dtype=torch.float32, bn=tile))
