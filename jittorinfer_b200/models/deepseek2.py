@@ -344,10 +344,11 @@ class DeepSeek2Model:
         dp = self.spec.dp_attention and self.spec.sharded
         base = self.expert_base if self.spec.expert_parallel else 0
         # the router launch of a decode batch also normalises its input rows and sorts the pairs by local expert
+        route = None if dp else ops.ExpertRoute(base, L.w_gate_exps.shape[0])
         ids, wts, g = ops.moe_gate(residual, L.w_router, L.router_bias, hp.n_expert_used, hp.n_group, hp.topk_group,
                                    hp.expert_weights_scale, hp.expert_weights_norm, hp.expert_gating_func == "sigmoid",
                                    L.n_shared_merged or 0, hp.group_score_top2,
-                                   route=None if dp else (base, L.w_gate_exps.shape[0]), pre_norm=(L.ffn_norm, hp.rms_eps))
+                                   route=route, pre_norm=(L.ffn_norm, hp.rms_eps))
         if dp:
             shared = None
             if L.w_gate_sh is not None:
@@ -357,12 +358,12 @@ class DeepSeek2Model:
             if getattr(self.comm, "fused_combine", False) and self.comm.fused and g.is_cuda and g.shape[0] <= self.comm.max_rows:
                 # decode batches: combine, all-reduce, residual (and the next block's norm) in one launch
                 return self.comm.moe_ffn_all_reduce(g, residual, ids, wts, L.w_gate_exps, L.w_up_exps, L.w_down_exps, L.w_gate_sh,
-                                                    L.w_up_sh, L.w_down_sh, base, hp.n_expert, norm)
+                                                    L.w_up_sh, L.w_down_sh, base, hp.n_expert, norm, route)
             part = ops.moe_ffn(g, None, ids, wts, L.w_gate_exps, L.w_up_exps, L.w_down_exps, L.w_gate_sh, L.w_up_sh,
-                               L.w_down_sh, base, n_expert=hp.n_expert)
+                               L.w_down_sh, base, n_expert=hp.n_expert, route=route)
             return self.comm.all_reduce(part, residual)
         return ops.moe_ffn(g, residual, ids, wts, L.w_gate_exps, L.w_up_exps, L.w_down_exps, L.w_gate_sh, L.w_up_sh,
-                           L.w_down_sh, base, n_expert=hp.n_expert, norm=norm)
+                           L.w_down_sh, base, n_expert=hp.n_expert, norm=norm, route=route)
 
     def _forward_sp(self, batch: ForwardBatch, kv_cache) -> torch.Tensor:
         """Tensor-parallel forward with a sequence-parallel residual stream (large prefill batches): every rank keeps

@@ -393,8 +393,9 @@ class NibalixModel:
         return ops.v_up(o_lat, L.w_uv)
 
     def _experts(self, L: _Layer, e: Experts, h: torch.Tensor):
-        ids, wts = ops.moe_gate(h, L.router, None, e.top, 1, 1, 1.0, True, False, route=(0, L.w_up_exps.shape[0]), logit_bias=L.router_b)
-        y, dest = ops.moe_routed(h, ids, wts, L.w_gate_exps, L.w_up_exps, L.w_down_exps)
+        route = ops.ExpertRoute(0, L.w_up_exps.shape[0])
+        ids, wts = ops.moe_gate(h, L.router, None, e.top, 1, 1, 1.0, True, False, route=route, logit_bias=L.router_b)
+        y, dest = ops.moe_routed(h, ids, wts, L.w_gate_exps, L.w_up_exps, L.w_down_exps, route)
         return y, dest, wts
 
     @torch.no_grad()

@@ -428,8 +428,9 @@ class RupatarModel:
 
     def _ff(self, L: _Layer, m: Experts, h: torch.Tensor) -> Dict[str, Any]:
         """The feed-forward's part of ``ops.scaled_update``'s arguments."""
-        ids, wts = ops.moe_gate(h, L.router, None, m.top, 1, 1, 1.0, False, True, L.n_merged, route=(0, L.w_up_exps.shape[0]))
-        y, dest = ops.moe_routed(h, ids, wts, None, L.w_up_exps, L.w_down_exps)
+        sort = ops.ExpertRoute(0, L.w_up_exps.shape[0])
+        ids, wts = ops.moe_gate(h, L.router, None, m.top, 1, 1, 1.0, False, True, L.n_merged, route=sort)
+        y, dest = ops.moe_routed(h, ids, wts, None, L.w_up_exps, L.w_down_exps, sort)
         out: Dict[str, Any] = {"moe": (y, dest, None)}
         if m.shared is not None and not L.n_merged:
             out["dense"] = ops.linear(ops.linear(h, L.w_up_sh, unary=("gelu",)), L.w_down_sh)

@@ -449,9 +449,9 @@ class ZomavikModel:
         """The feed-forward's part of ``ops.scaled_update``'s arguments."""
         if isinstance(m, Dense):
             return {"dense": ops.linear(ops.linear(h, L.w_up, unary=("relu2",)), L.w_down)}
-        route = ops.moe_gate(h, L.router, None, m.top, m.groups, m.keep, 1.0, True, False, L.n_merged, route=(0, L.w_up_exps.shape[0]),
-                             shared_gate=m.shared is not None)
-        y, dest = ops.moe_routed(h, route[0], route[1], L.w_gate_exps, L.w_up_exps, L.w_down_exps)
+        sort = ops.ExpertRoute(0, L.w_up_exps.shape[0])
+        route = ops.moe_gate(h, L.router, None, m.top, m.groups, m.keep, 1.0, True, False, L.n_merged, route=sort, shared_gate=m.shared is not None)
+        y, dest = ops.moe_routed(h, route[0], route[1], L.w_gate_exps, L.w_up_exps, L.w_down_exps, sort)
         out: Dict[str, Any] = {"moe": (y, dest, route[1])}
         if m.shared is not None and not L.n_merged:
             out["dense"], out["dense_gate"] = ops.linear(ops.gateup(h, L.w_gate_sh, L.w_up_sh, "silu"), L.w_down_sh), route[2]

@@ -13,6 +13,7 @@ import os
 import torch
 
 from . import reference as ref
+from .specs import ExpertRoute
 
 _FORCE_TORCH = os.environ.get("JITTORINFER_OPS", "").lower() == "torch"
 _native = None
@@ -132,7 +133,7 @@ def moe_gate(g, w_router, bias, k, n_group, topk_group, scale, norm, sigmoid, n_
              logit_bias=None, shared_gate=False):
     """``w_router`` fp32, or bf16 with bf16 activations (products of exact operands on the tensor cores, fp32 sums).  ``shared_gate``: the last row of ``w_router`` is the shared experts' gate, not an expert: their weight is its sigmoid (``n_shared``
     columns), and the router outputs' last column is returned as well.
-    ``route=(expert_base, E_local)`` tells the CUDA path which local expert sort follows (see ``native.moe_gate``).
+    ``route`` (an ``ExpertRoute``, or (expert_base, E_local)) tells the CUDA path which local expert sort follows (see ``native.moe_gate``).
     ``pre_norm=(weight, eps)``: ``g`` is the un-normalised block input; returns (ids, wts, rmsnorm(g) * weight) -- on the CUDA
     path the router launch of a decode batch normalises the rows itself."""
     if use_native(g):
@@ -144,10 +145,13 @@ def moe_gate(g, w_router, bias, k, n_group, topk_group, scale, norm, sigmoid, n_
     return ref.moe_gate(g, w_router, bias, k, n_group, topk_group, scale, norm, sigmoid, n_shared, group_top2, logit_bias, shared_gate)
 
 
-def moe_routed(x, ids, wts, wg, wu, wd):
+def moe_routed(x, ids, wts, wg, wu, wd, route=None):
     """(expert outputs of the (token, choice) pairs, row of each pair); the weighted sum is the caller's (``block_update``).  ``wg`` None: experts
-    without a gate, gelu(w x up^T) down^T -- the weight multiplies their input, the sum of the outputs is the result."""
-    return (nat() if use_native(x) else ref).moe_routed(x, ids, wts, wg, wu, wd)
+    without a gate, gelu(w x up^T) down^T -- the weight multiplies their input, the sum of the outputs is the result.  ``route``: the ``ExpertRoute``
+    given to the ``moe_gate`` call whose ids and weights these are, unchanged since."""
+    if use_native(x):
+        return nat().moe_routed(x, ids, wts, wg, wu, wd, route=route)
+    return ref.moe_routed(x, ids, wts, wg, wu, wd)
 
 
 def moe_experts(x, ids, wts, wg, wu, wd, expert_base=0):
@@ -156,11 +160,11 @@ def moe_experts(x, ids, wts, wg, wu, wd, expert_base=0):
     return ref.moe_experts(x, ids, wts, wg, wu, wd, expert_base)
 
 
-def moe_ffn(x, residual, ids, wts, wg, wu, wd, wgs, wus, wds, expert_base=0, n_expert=None, norm=None):
-    """``n_expert``: size of the router's expert set (lets the CUDA path estimate how many local experts a batch hits).
+def moe_ffn(x, residual, ids, wts, wg, wu, wd, wgs, wus, wds, expert_base=0, n_expert=None, norm=None, route=None):
+    """``n_expert``: size of the router's expert set (lets the CUDA path estimate how many local experts a batch hits).  ``route``: see ``moe_routed``.
     ``norm=(weight, eps)``: returns (out, rmsnorm(out) * weight) -- the CUDA path computes both in the combine launch."""
     if use_native(x) and x.dtype == torch.bfloat16:
-        return nat().moe_ffn(x, residual, ids, wts, wg, wu, wd, wgs, wus, wds, expert_base, n_expert, norm)
+        return nat().moe_ffn(x, residual, ids, wts, wg, wu, wd, wgs, wus, wds, expert_base, n_expert, norm, route)
     out = ref.moe_ffn(x, residual, ids, wts, wg, wu, wd, wgs, wus, wds, expert_base)
     return (out, ref.rmsnorm(out, norm[0], norm[1])[0]) if norm is not None else out
 

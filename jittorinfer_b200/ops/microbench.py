@@ -75,6 +75,7 @@ def main(argv=None):
     ap.add_argument("--torch", action="store_true", help="time the PyTorch/cuBLAS op instead (baseline)")
     a = ap.parse_args(argv)
     from . import native as nat
+    from .specs import ExpertRoute
     nat.load()
     dev = "cuda"
     g = torch.Generator(device=dev).manual_seed(0)
@@ -175,19 +176,22 @@ def main(argv=None):
         report(f"prefill attention op (gather + K/V expansion + kernel) T={T} H={H}", ms, 0, flops + 2.0 * T * 512 * H * 256)
         nat.check_status()
     elif a.case == "route":
-        # router chain of one MoE layer: logits + gating + expert sort as three launches vs the one-launch kernel
+        # router chain of one MoE layer: logits, gating and expert sort as three launches, gate and sort as one, all as one
         E, k, d, T = a.E, a.k, a.d, a.T
         gx = rnd(T, d)
         wr = torch.randn(E, d, device=dev, generator=g) * 0.05
-        for fused in (False, True):
-            nat.FUSED_ROUTE = fused
+        for form in ("three launches", "two launches", "one launch"):
+            nat.FUSED_ROUTE = form == "one launch"
+            if T > {"three launches": T, "two launches": nat.GATE_SORT_MAX_T, "one launch": nat.FUSED_ROUTE_MAX_T}[form]:
+                continue
 
             def fn():
-                ids, wts = nat.moe_gate(gx, wr, None, k, 1, 1, 1.0, False, False, 0, False, (0, E))
-                return nat.moe_permute(ids, 0, E)
+                route = ExpertRoute(0, E) if form != "three launches" else None
+                ids, wts = nat.moe_gate(gx, wr, None, k, 1, 1, 1.0, False, False, 0, False, route)
+                return route.pairs if route is not None else nat.moe_permute(ids, 0, E)
 
             ms = timeit(fn, a.iters, a.warmup)
-            report(f"route T={T} E={E} k={k} d={d} " + ("one launch" if fused else "three launches"), ms, E * d * 4 + T * d * 2, 2.0 * T * E * d)
+            report(f"route T={T} E={E} k={k} d={d} {form}", ms, E * d * 4 + T * d * 2, 2.0 * T * E * d)
     elif a.case == "combine_norm":
         # expert combine followed by the next block's RMSNorm: two launches vs one
         k, d, T = a.k, a.d, a.T

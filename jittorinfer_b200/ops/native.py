@@ -12,7 +12,7 @@ from typing import Dict, Optional
 
 import torch
 
-from .specs import RowNorms
+from .specs import ExpertRoute, RowNorms
 
 _lib = None
 _ws: Dict[int, "Workspace"] = {}
@@ -556,11 +556,15 @@ def mha_prefill(q, cache, w_kv_b, block_tables, seq_lens, q_start, scale, n_head
 # ---- MoE -----------------------------------------------------------------------------------------
 def moe_gate(g, w_router, bias, k, n_group, topk_group, scale, norm, sigmoid, n_shared=0, group_top2=False, route=None,
              pre_norm=None, logit_bias=None, shared_gate=False):
-    """``route=(expert_base, E_local)``: the caller will sort these ids by local expert next (``moe_permute``, ``moe_routed``); for decode
-    batches the gate and the sort then run as one launch, whose result travels with ``ids``.
+    """``route``: the caller will sort these ids by local expert next.  An ``ExpertRoute``, for ``moe_routed``: for decode batches the gate and
+    the sort run as one launch, whose result the route then holds.  (expert_base, E_local), for ``moe_permute``: only the opt-in launch of
+    router, gate and sort (``FUSED_ROUTE``) sorts ahead.
     ``pre_norm=(weight, eps)``: ``g`` holds un-normalised rows; returns (ids, wts, rmsnorm(g) * weight), the norm done by
     the router launch itself for decode batches."""
     T, d = g.shape
+    handed = route if isinstance(route, ExpertRoute) else None
+    if handed is not None:
+        handed.pairs, route = None, (handed.base, handed.n_local)
     fused = FUSED_ROUTE and route is not None and T <= FUSED_ROUTE_MAX_T and logit_bias is None and not shared_gate and g.dtype == torch.bfloat16
     g_in = g
     g_pre = None
@@ -589,15 +593,18 @@ def moe_gate(g, w_router, bias, k, n_group, topk_group, scale, norm, sigmoid, n_
                                        T, d, E, k, n_group, topk_group, float(scale), int(norm), int(sigmoid), n_shared,
                                        int(group_top2), expert_base, E_local, pre_norm_k[0].data_ptr() if pre_norm_k is not None else None,
                                        float(pre_norm_k[1]) if pre_norm_k is not None else 0.0, _p(g_out), _stream()), "moe_route_fused")
-        _route_stash.clear()                       # at most one pending result: the sort that follows this gate
-        _route_stash[(ids.data_ptr(), expert_base, E_local)] = (seg, src, dest, ids)
+        if handed is not None:
+            handed.pairs = (seg, src, dest, None)
+        else:
+            _route_stash.clear()                   # at most one pending result: the sort that follows this gate
+            _route_stash[(ids.data_ptr(), expert_base, E_local)] = (seg, src, dest, ids)
         return (ids, wts, g_out if g_out is not None else g_pre) if pre_norm is not None else (ids, wts)
     own = g.dtype == torch.bfloat16 and not by_gemm and d % 8 == 0 and d <= 8192      # the router kernel; else fp32 products of the library
     if by_gemm:
         gemm(g, w_router, out=logits)
     elif not own:
         torch.matmul(g.float(), w_router.T, out=logits)
-    if route is not None and 0 < T <= GATE_SORT_MAX_T and not ids.is_inference():
+    if handed is not None and 0 < T <= GATE_SORT_MAX_T:
         expert_base, E_local = route
         n = T * (k + n_shared)
         seg = torch.empty(2 * E_local + 1, dtype=torch.int32, device=g.device)[:E_local + 1]     # + room for the list of experts hit
@@ -606,24 +613,12 @@ def moe_gate(g, w_router, bias, k, n_group, topk_group, scale, norm, sigmoid, n_
                                      wts.data_ptr(), T, d, E, k, n_group, topk_group, float(scale), int(norm), int(sigmoid), n_shared, int(group_top2),
                                      int(shared_gate), expert_base, E_local, seg.data_ptr(), src.data_ptr(), dest.data_ptr(), row_wts.data_ptr(),
                                      _stream()), "moe_gate")
-        ids.sorted_pairs = (expert_base, E_local, ids._version, seg, src, dest)
-        wts.sorted_pairs = (ids.data_ptr(), wts._version, row_wts)
+        handed.pairs = (seg, src, dest, row_wts)
         return (ids, wts) + ((g,) if pre_norm is not None else ()) + ((logits[:, E],) if shared_gate else ())
     _ck(load().jib_moe_gate(g.data_ptr() if own else None, w_router.data_ptr(), _p(bias), _p(logit_bias), logits.data_ptr(), ids.data_ptr(), wts.data_ptr(), T, d,
                             E, k, n_group, topk_group, float(scale), int(norm), int(sigmoid), n_shared, int(group_top2), int(shared_gate), _stream()),
         "moe_gate")
     return (ids, wts) + ((g,) if pre_norm is not None else ()) + ((logits[:, E],) if shared_gate else ())
-
-
-def _sorted_by_gate(ids, expert_base, E_local):
-    """(seg, src, dest) of ids that a gate launch sorted for these experts and that nobody has written to since, else None."""
-    r = getattr(ids, "sorted_pairs", None)
-    return r[3:] if r is not None and r[:3] == (expert_base, E_local, ids._version) else None
-
-
-def _row_weights_of_gate(ids, wts):
-    r = getattr(wts, "sorted_pairs", None)
-    return r[2] if r is not None and r[:2] == (ids.data_ptr(), wts._version) else None
 
 
 def moe_permute(ids, expert_base, E_local, wts=None, row_wts=None):
@@ -633,9 +628,6 @@ def moe_permute(ids, expert_base, E_local, wts=None, row_wts=None):
     hit = _route_stash.pop((ids.data_ptr(), expert_base, E_local), None)
     if hit is not None and hit[3] is ids and row_wts is None:          # the fused router launch already sorted exactly these ids
         return hit[0], hit[1], hit[2]
-    hit = _sorted_by_gate(ids, expert_base, E_local)
-    if hit is not None and row_wts is None:
-        return hit
     seg = torch.empty(2 * E_local + 1, dtype=torch.int32, device=dev)[:E_local + 1]       # + room for the list of experts hit
     src = torch.empty(T * k, dtype=torch.int32, device=dev)
     dest = torch.empty(T, k, dtype=torch.int32, device=dev)
@@ -693,13 +685,21 @@ def expected_active_experts(T: int, k: int, E_local: int, n_expert: int) -> int:
     return max(1, min(E_local, always + int(routed_local * p_hit + 0.999)))
 
 
-def moe_routed(x, ids, wts, wg, wu, wd, expert_base=0, n_expert=None):
+def moe_routed(x, ids, wts, wg, wu, wd, expert_base=0, n_expert=None, route=None):
     """Expert-sorted rows -> grouped gate|up GEMM (SiLU*mul epilogue) -> grouped down GEMM.  ``wg`` None: the first product is wu's alone, its
-    epilogue gelu(weight of the row * product).  Returns (y [T*k, d] in sorted order, dest [T,k])."""
+    epilogue gelu(weight of the row * product).  ``route``: the ``ExpertRoute`` of the gate call that gave these ids and weights, neither
+    changed since.  Returns (y [T*k, d] in sorted order, dest [T,k])."""
     T, k = ids.shape
     E_local = wu.shape[0]
-    fn = _row_weights_of_gate(ids, wts) if wg is None and _sorted_by_gate(ids, expert_base, E_local) is not None else None
-    if fn is not None or wg is not None:
+    pairs = route.pairs if route is not None else None
+    if pairs is not None and ((route.base, route.n_local) != (expert_base, E_local) or pairs[2].shape != ids.shape):
+        raise ValueError(f"route of {tuple(pairs[2].shape)} pairs over experts {route.base} + {route.n_local} for {tuple(ids.shape)} pairs over {expert_base} + {E_local}")
+    fn = None
+    if pairs is not None and (wg is not None or pairs[3] is not None):
+        seg, src, dest = pairs[:3]
+        if wg is None:
+            fn = pairs[3]
+    elif wg is not None:
         seg, src, dest = moe_permute(ids, expert_base, E_local)
     else:
         fn = torch.empty(T * k, dtype=torch.float32, device=x.device)
@@ -749,10 +749,10 @@ def moe_experts(x, ids, wts, wg, wu, wd, expert_base=0):
     return moe_combine(y, dest, wts, None, None).float()
 
 
-def moe_ffn(x, residual, ids, wts, wg, wu, wd, wgs, wus, wds, expert_base=0, n_expert=None, norm=None):
+def moe_ffn(x, residual, ids, wts, wg, wu, wd, wgs, wus, wds, expert_base=0, n_expert=None, norm=None, route=None):
     """residual + shared_experts(x) + sum_k w_k expert_k(x), bf16; residual/shared may be None.
-    ``norm=(weight, eps)``: returns (out, rmsnorm(out) * weight), the norm computed by the combine launch."""
-    y, dest = moe_routed(x, ids, wts, wg, wu, wd, expert_base, n_expert)
+    ``norm=(weight, eps)``: returns (out, rmsnorm(out) * weight), the norm computed by the combine launch.  ``route``: see ``moe_routed``."""
+    y, dest = moe_routed(x, ids, wts, wg, wu, wd, expert_base, n_expert, route)
     shared = None
     if wgs is not None:
         shared = gemm(gemm(x, wgs, wus), wds)

@@ -2,9 +2,20 @@
 from __future__ import annotations
 
 from dataclasses import dataclass
-from typing import Optional
+from typing import Optional, Tuple
 
 import torch
+
+
+class ExpertRoute:
+    """Experts ``base`` .. ``base + n_local - 1``, whose products follow a gate call.  The caller makes one per gate call and gives it to the
+    ``moe_gate`` and to the ``moe_routed`` or ``moe_ffn`` that belong together; ids and weights stay as they are in between.  ``pairs``: what the gate
+    launch sorted on the way, (seg, src, dest, weights in sorted order or None), or None.  They belong to the gate's stream."""
+    __slots__ = ("base", "n_local", "pairs")
+
+    def __init__(self, base: int, n_local: int):
+        self.base, self.n_local = base, n_local
+        self.pairs: Optional[Tuple[Optional[torch.Tensor], ...]] = None
 
 
 @dataclass

@@ -266,14 +266,14 @@ class FusedCommunicator(Communicator):
     # 4.90 -> 4.80 ms on 2 GPUs, 7.25 -> 6.99 ms on 4, 12.34 -> 11.50 ms on 8.
     fused_combine = os.environ.get("JIB_FUSED_COMBINE_AR", "0") == "1"
 
-    def moe_ffn_all_reduce(self, x, residual, ids, wts, wg, wu, wd, wgs, wus, wds, expert_base, n_expert=None, norm=None):
+    def moe_ffn_all_reduce(self, x, residual, ids, wts, wg, wu, wd, wgs, wus, wds, expert_base, n_expert=None, norm=None, route=None):
         """residual + all-reduce(local experts' weighted sum + this rank's shard of the shared experts) for a decode
         batch; ``norm=(weight, eps)`` adds rmsnorm(result) * weight -> (out, normed).  One launch after the expert GEMMs
         instead of combine, all-reduce and norm."""
         T, d = x.shape
         site = self._next_site()
         nat = self.native
-        y, dest = nat.moe_routed(x, ids, wts, wg, wu, wd, expert_base, n_expert)
+        y, dest = nat.moe_routed(x, ids, wts, wg, wu, wd, expert_base, n_expert, route)
         shared = nat.gemm(nat.gemm(x, wgs, wus), wds) if wgs is not None else None
         out = torch.empty(T, d, dtype=torch.bfloat16, device=x.device)
         normed = torch.empty(T, d, dtype=torch.bfloat16, device=x.device) if norm is not None else None

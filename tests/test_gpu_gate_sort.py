@@ -2,6 +2,8 @@
 import pytest
 import torch
 
+from jittorinfer_b200.ops import ExpertRoute
+
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
@@ -50,23 +52,21 @@ def test_one_launch(nat, T, E, k, n_shared, n_group, topk_group, top2, sigmoid, 
     lb = torch.randn(E, generator=gen, device=DEV) if n_group == 1 and E != 64 else None
     args = (x, w, bias, k, n_group, topk_group, 2.5, norm, sigmoid, n_shared, top2)
     ids0, wts0 = nat.moe_gate(*args, logit_bias=lb)
+    route = ExpertRoute(base, E_local)
     for _ in range(2):
-        ids, wts = nat.moe_gate(*args, route=(base, E_local), logit_bias=lb)
+        ids, wts = nat.moe_gate(*args, route=route, logit_bias=lb)
     assert torch.equal(ids, ids0) and torch.equal(wts, wts0)
-    seg, src, dest = nat.moe_permute(ids, base, E_local)
-    order = check_sort(ids, base, E_local, seg, src, dest)
-    if T <= nat.GATE_SORT_MAX_T:
-        assert src.data_ptr() == ids.sorted_pairs[4].data_ptr()               # the gate's own
-        rows = nat._row_weights_of_gate(ids, wts)
+    assert (route.pairs is None) == (T > nat.GATE_SORT_MAX_T)
+    if route.pairs is not None:
+        seg, src, dest, rows = route.pairs
+        order = check_sort(ids, base, E_local, seg, src, dest)
         assert torch.equal(rows[:len(order)].cpu(), wts.flatten().cpu()[order])
-        assert nat.moe_permute(ids, base, E_local - 1)[1].data_ptr() != src.data_ptr()
-        ids += 0                                                              # written to: sorted anew
-        assert nat._sorted_by_gate(ids, base, E_local) is None
-        wts.mul_(2)
-        assert nat._row_weights_of_gate(ids, wts) is None
-    with torch.inference_mode():                                              # no version counters: the two launches
-        ids, wts = nat.moe_gate(*args, route=(base, E_local), logit_bias=lb)
-        assert torch.equal(ids, ids0) and not hasattr(ids, "sorted_pairs")
+    check_sort(ids, base, E_local, *nat.moe_permute(ids, base, E_local))
+    with torch.inference_mode():
+        ids, wts = nat.moe_gate(*args, route=route, logit_bias=lb)
+        assert torch.equal(ids, ids0) and (route.pairs is None or torch.equal(route.pairs[2], dest))
+    # a pair instead of a route: gate and sort stay apart
+    assert torch.equal(nat.moe_gate(*args, route=(base, E_local), logit_bias=lb)[0], ids0)
 
 
 def test_no_numbers_and_infinities(nat):
