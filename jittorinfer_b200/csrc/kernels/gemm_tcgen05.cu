@@ -868,13 +868,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             if (!ptile_decode<BN>(args, item, n_x, n_y, t)) continue;
             const int buf = j & 1;
             if (!mbar_wait(&acc_ready[buf], (j >> 1) & 1)) { jib_report(args.status, JIB_ERR_WAIT_TIMEOUT, 14, item); ok = false; }
-            {
-                // the four warps leave together or not at all: they meet at named barrier 1 inside the tile
-                uint32_t all;
-                asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                             : "=r"(all) : "r"((uint32_t) ok) : "memory");
-                ok = all != 0;
-            }
+            ok = all_of_128(ok);      // the four warps leave together or not at all: they meet at named barrier 1 inside the tile
             if (!ok) break;
             tc_fence_after();
             const uint32_t tbase = tmem + buf * C::ACC_COLS + ((uint32_t) (q * 32) << 16);

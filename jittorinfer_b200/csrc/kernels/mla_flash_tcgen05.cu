@@ -104,7 +104,6 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     uint64_t * p_ready = s_ready + 1;
     uint64_t * o_ready = p_ready + 1;
     uint32_t * tmem_slot = (uint32_t *) (o_ready + 1);
-    volatile int * failed = (volatile int *) (tmem_slot + 1);    // a softmax warp gave up on a wait: the four leave together
 
     // ---- work description: up to QT distinct sequences among this CTA's tokens ("passes") ----
     // pass j covers the tokens of the group that belong to sequence pass_seq[j]; a column of another sequence is
@@ -172,7 +171,6 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (threadIdx.x == 0) {
         for (int i = 0; i < C::NPAIR; ++i) { mbar_init(&lat_full[i], 1); mbar_init(&lat_free[i], 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(&rope_full[i], 1); mbar_init(&rope_free[i], 1); }
-        *failed = 0;
         mbar_init(q_full, 1);
         mbar_init(s_ready, 1);
         mbar_init(p_ready, 4);
@@ -328,7 +326,8 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         while (true) {
             const bool dry = it < 0;
             if (!dry) {
-                if (!mbar_wait(s_ready, it & 1)) { jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 27, it); ok = false; *failed = 1; }
+                ok = __all_sync(0xffffffffu, mbar_wait(s_ready, it & 1));      // one answer per warp: warp-wide instructions follow
+                if (!ok) jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 27, it);
                 tc_fence_after();
                 if (it == 0) JIB_KS_T(2, 4, 64);
             }
@@ -377,7 +376,8 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             }
             // running-max correction of O^T (previous PV products must have landed)
             if (it > 0 && ok) {
-                if (!mbar_wait(o_ready, (it - 1) & 1)) { jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 28, it); ok = false; *failed = 1; }
+                ok = __all_sync(0xffffffffu, mbar_wait(o_ready, (it - 1) & 1));
+                if (!ok) jib_report(a.status, JIB_ERR_WAIT_TIMEOUT, 28, it);
                 tc_fence_after();
                 if (any_corr && ok) {
 #pragma unroll 1
@@ -398,8 +398,10 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             tc_fence_before();
             __syncwarp();
             if (lane == 0 && !dry && ok) mbar_arrive(p_ready);
-            asm volatile("bar.sync 1, 128;" ::: "memory");   // red[] reuse in the next tile
-            if (*failed) break;
+            // red[] reuse in the next tile.  A warp that gave up on a wait takes the others along in the same barrier: a word in shared memory
+            // could be written by a warp that is a tile ahead before a slow one has read it, which would then leave the others at the next barrier.
+            ok = all_of_128(ok);
+            if (!ok) break;
             // ---- next tile: the next one of this pass, the first of the next pass with any, or the results ----
             bool last = dry;
             if (!dry) {

@@ -104,6 +104,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t * bar, uint32_t parity) {
     return false;
 }
 
+// Named barrier 1 of four warps, and their decision: true when `ok` is for every thread.
+__device__ __forceinline__ bool all_of_128(bool ok) {
+    uint32_t all;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(all) : "r"((uint32_t) ok) : "memory");
+    return all != 0;
+}
+
 // ---- TMA --------------------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap * m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");

@@ -16,6 +16,7 @@ another call site or another step is a protocol bug.  The programs mirror the ke
 What the model cannot show is memory ordering inside one GPU (release/acquire, proxy fences): that is by construction
 in the kernels (``st.release.sys`` after ``__threadfence_system``, ``ld.acquire.sys`` before the loads).
 """
+import pathlib
 import random
 
 import pytest
@@ -512,3 +513,57 @@ def test_decode_attention_pipeline_never_reads_a_tile_out_of_turn(n_tiles, npair
     for seed in range(40):
         for bias in (None, 0, 1, 2):
             _PhaseSim(_flash_roles(n_tiles, npair), seed, bias).run()
+
+
+# ---- leaving early: the four softmax warps of mla_flash_kernel when one of them gives up on a bounded wait ------------------------------
+# A tile is: wait for the scores, a barrier, wait for the last value product, a barrier behind which all leave or all go on.  ``expiry``: (warp,
+# tile, first or second wait) that runs out.  ``vote``: the second barrier itself carries the decision (bar.red); else a word beside it does.
+def _leaving_warps(n_tiles, expiry, vote, n_warps=4):
+    def meet(w, at, ok):
+        yield ("store", ("here", at, w), ok)
+        yield ("wait", lambda mem: all(("here", at, v) in mem for v in range(n_warps)))
+
+    def read(key, into):
+        yield ("wait", lambda mem: into.append(mem.get(key)) or True)
+
+    def warp(w):
+        for t in range(n_tiles):
+            ok = True
+            for n in (0, 1):
+                if ok and (w, t, n) == expiry:
+                    ok = False
+                    yield ("store", "failed", True)
+                yield from meet(w, (t, n), ok)
+            if vote:
+                all_ok = []
+                for v in range(n_warps):
+                    yield from read(("here", (t, 1), v), all_ok)
+                if not all(x is not False for x in all_ok):
+                    return
+            else:
+                seen = []
+                yield from read("failed", seen)
+                if seen[-1]:
+                    return
+    return [warp(w) for w in range(n_warps)]
+
+
+@pytest.mark.parametrize("expiry", [None, (0, 0, 0), (2, 0, 1), (1, 1, 0), (3, 2, 1)])
+def test_softmax_warps_leave_together(expiry):
+    for seed in range(200):
+        Sim(_leaving_warps(4, expiry, True), seed, bias=None if seed % 2 else seed % 4).run()
+
+
+def test_the_model_catches_a_word_beside_the_barrier():
+    """A fast warp gives up in the next tile before a slow one has read the word: the slow one leaves alone, the others stand at a barrier."""
+    with pytest.raises(AssertionError, match="deadlock"):
+        for seed in range(400):
+            Sim(_leaving_warps(4, (0, 1, 0), False), seed, bias=0).run()
+
+
+def test_the_kernel_leaves_by_vote():
+    src = (pathlib.Path(__file__).parents[1] / "jittorinfer_b200/csrc/kernels/mla_flash_tcgen05.cu").read_text()
+    softmax = src[src.index("while (true) {"):src.index("tmem_dealloc")]
+    assert "ok = all_of_128(ok);\n            if (!ok) break;" in softmax and "failed" not in softmax
+    # waits whose answer decides over warp-wide instructions are answered per warp
+    assert softmax.count("ok = __all_sync(0xffffffffu, mbar_wait(") == 2
