@@ -62,6 +62,7 @@ struct FlashArgs {
     int * status;
     int max_blocks, n_seqs, T, H, n_splits, n_blocks;
     int window;           // > 0: position i sees j with 0 <= i - j < window
+    int warm;             // this many of the first CTAs make a dry pass (see the softmax warps)
     float scale_log2e;
 };
 
@@ -318,11 +319,19 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         bool ok = true;
         // A decode CTA runs this code once or twice per launch, and a dozen other kernels between two launches push it out of the
         // instruction cache: with the first real tile as the first pass, scores to results took 10 us.  So tile -1 is a dry pass over
-        // whatever the buffers hold, while the previous kernel still runs: no waits, no arrivals, no global stores.  For the same reason
+        // whatever the buffers hold, while the previous kernel still runs: no waits, no arrivals, no global stores.  The first CTA of each
+        // SM makes it; later ones find the code there.  For the same reason
         // the bodies are short (a maximum over a warp is one instruction, 16 columns are added up in 16 exchanges).  From the previous
         // kernel's end to this one's inside a decode graph, 16 heads: 8 sequences of 1040 rows 11.6 -> 8.0 us; one of up to 64 rows, in
         // one split, 13.7 and 3.0 us for the merge -> 10.3 us.  What is left is a chain: query and rows in (3 us), two products, results.
-        int it = -1, p = 0, kb = 0;
+        const bool warm = QT == 1 && (int) (blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)) < a.warm;
+        int it = warm ? -1 : 0, p = 0, kb = 0;
+        auto begin = [&] {
+            while (pass_k1[p] <= pass_k0[p]) ++p;               // total_tiles > 0: there is one
+            kb = pass_k0[p];
+            pdl_wait();
+        };
+        if (!warm) begin();
         while (true) {
             const bool dry = it < 0;
             if (!dry) {
@@ -486,10 +495,7 @@ mla_flash_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 }
                 if (!dry) break;
                 asm volatile("bar.sync 1, 128;" ::: "memory");      // red[]
-                p = 0;
-                while (pass_k1[p] <= pass_k0[p]) ++p;               // total_tiles > 0: there is one
-                kb = pass_k0[p];
-                pdl_wait();
+                begin();
             }
             ++it;
         }
@@ -568,6 +574,7 @@ extern "C" JIB_EXPORT int jib_mla_flash(const void * q, const void * cache, long
     a.o_lat = (bf16 *) o_lat; a.status = status; a.max_blocks = max_blocks; a.n_seqs = n_seqs; a.T = T; a.H = H;
     a.n_splits = n_splits; a.n_blocks = (int) (n_slots / BLK); a.window = window;
     a.scale_log2e = scale * 1.4426950408889634f;
+    a.warm = qt == 1 && jib::warm_enabled() ? jib::sm_count() : 0;
     dim3 grid((T + qt - 1) / qt, n_splits, (H + 15) / 16);
     return qt == 1 ? launch_flash<1>(mq, mkv, a, grid, stream) : launch_flash<2>(mq, mkv, a, grid, stream);
 }

@@ -45,17 +45,18 @@ def close(a, b):
 
 
 # one row, around the 16-row steps of the value product, a block of 64 and a tile of 128; table rows of exactly the needed width (fewest
-# splits) and much wider ones (most splits)
+# splits) and much wider ones (most splits); a window that ends inside a step, a block and a tile; more CTAs than SMs: past those with a dry pass
 @pytest.mark.parametrize("H", [16, 24, 128])
 @pytest.mark.parametrize("width", [None, 40])
-@pytest.mark.parametrize("lens", [[1], [15, 16, 17], [63, 64, 65], [127, 128, 129, 193], [0, 40], [2000]])
-def test_decode(nat, H, width, lens):
+@pytest.mark.parametrize("window", [0, 70])
+@pytest.mark.parametrize("lens", [[1], [15, 16, 17], [63, 64, 65], [127, 128, 129, 193], [0, 40], [2000], [1 + i * 7 % 200 for i in range(160)]])
+def test_decode(nat, H, width, window, lens):
     bt, rows = tables(lens, width=width)
     cache, q = rnd(rows, 576, seed=1), rnd(len(lens), H, 576, seed=2, scale=0.3)
     qs = i32(list(range(len(lens) + 1)))
     for _ in range(2):
-        o = nat.mla_attention(q, cache, bt, i32(lens), qs, 0.11, 512, 64, 1)
-    want = ref.mla_attention(q, cache, bt, i32(lens), qs, 0.11, 512, 64)
+        o = nat.mla_attention(q, cache, bt, i32(lens), qs, 0.11, 512, 64, 1, None, window)
+    want = ref.mla_attention(q, cache, bt, i32(lens), qs, 0.11, 512, 64, window)
     close(o[[i for i, n in enumerate(lens) if n]], want[[i for i, n in enumerate(lens) if n]])
     assert all(not bool(o[i].any()) for i, n in enumerate(lens) if n == 0)
 
