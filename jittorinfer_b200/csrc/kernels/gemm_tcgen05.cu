@@ -1051,15 +1051,19 @@ int auto_splits(long long base_ctas, int num_kb, int bn, int sms) {
     return splits;
 }
 
-// Token-tile width and split count of a plain product of more than 32 tokens: the cheapest pair by a cost model (us) whose constants are
-// a least-squares fit to 315 products x their pairs measured on a B200 (N 160..24576, K 512..16384, 17..2048 tokens, single and gated).
+// Token-tile width and split count of a plain product of more than 32 tokens: the cheapest pair by a cost model (us) whose constants were
+// fitted to products x their pairs measured on a B200; profiles/gemm_plan_products.csv has 439 products (N 512..24576, K 512..10944, 33..2048
+// tokens, single and gated, weights out of memory) under the rule before, under this one and under the best measured pair.
 // What they say: a CTA of one tile costs a start-up that grows with the tile and ~0.2 us per 64 of K (0.36 at 256 tokens), so ONE full
 // wave of small tiles beats half a wave of large ones; two narrow CTAs share an SM at 1.43x; a split costs ~2 us plus its partials;
-// persistent rounds cost less than waves.  Taking the power of two that covers the tokens instead leaves most SMs idle between 33 and
-// ~1000 tokens: 2048 x 2048 at 64 tokens 14.0 -> 7.0 us, at 777 58 -> 13.4 us, 3648 x 2048 at 333 57.9 -> 13.3 us; over all measured
-// shapes that rule is 1.60x the best pair on average, this one 1.02x.
+// persistent rounds cost less than waves.  CTAs run through all feature tiles before they come to the next token tile, so weights that L2
+// does not hold come out of memory once per token tile (24576 x 5120 at 33 tokens: 93 us in tiles of 16, 56 us in one of 64).  Taking the
+// power of two that covers the tokens instead leaves most SMs idle between 33 and ~1000 tokens: 2048 x 2048 at 64 tokens 14.0 -> 7.0 us, at
+// 777 58 -> 13.4 us.  Over the table that rule is 1.43x the best pair on average, this one 1.02x.
+// Gated pairs of 32-token tiles stay unsplit: their splits were nowhere the best pair (4 to 100 % behind tiles of 16 or 64).
 // Splits of wide tiles need whole SMs of one GPC: past `cap` CTAs the last clusters wait for a second wave (2112 x 5120 at 128 tokens,
-// 64-token tiles: 3 splits = 102 CTAs 16.8 us, 4 splits = 136 CTAs 25.4 us; narrow tiles, two per SM: 272 CTAs fit, 288 do not).
+// 64-token tiles: 3 splits = 102 CTAs 16.8 us, 4 splits = 136 CTAs 25.4 us; gated 2816 x 5120 at 77, 128-token tiles: 6 splits = 132 CTAs 19.5 us;
+// narrow tiles, two per SM: 272 CTAs fit, 288 do not).
 struct TilePlan {
     int bn, splits;
 };
@@ -1069,16 +1073,19 @@ TilePlan plan_tiles(int N, int K, int T, bool dual, bool can_persist, int sms) {
     const double gate_kb = dual ? 2.7 : 1.0;                      // per 64 of K of a gated pair
     const int n_tiles = (N + BM - 1) / BM, num_kb = (K + BK - 1) / BK;
     const double weights = (double) N * K * (dual ? 4 : 2);
+    // share of them that L2 has lost when the next token tile comes: none up to 70 MB, all from 140 MB on
+    const double lost = weights < 70e6 ? 0. : weights > 140e6 ? 1. : weights / 70e6 - 1.;
     TilePlan best = {0, 1};
     double best_us = 1e30;
     for (int i = 0; i < (dual ? 4 : 5); ++i) {
         const int bn = 16 << i, occ = bn <= 32 ? 2 : 1;
-        const long long tiles = (long long) n_tiles * ((T + bn - 1) / bn);
+        const int t_tiles = (T + bn - 1) / bn;
+        const long long tiles = (long long) n_tiles * t_tiles;
         const double l2_us = 3.0 + (double) tiles * num_kb * (BK * 2) * (BM * (dual ? 2 : 1) + bn) / 18.2e6;
-        const double hbm_us = 3.0 + (weights + 2.0 * T * ((double) K + N)) / 4.26e6;
+        const double hbm_us = 3.0 + (weights * (1. + (t_tiles - 1) * lost) + 2.0 * T * ((double) K + N)) / 4.7e6;
         for (int s = 1; s <= 8; ++s) {
             if (s > 1 && (s > num_kb / 4 || (dual && bn == 32))) break;
-            const int cap = occ == 2 ? sms * (s < 8 ? 184 : 173) / 100 : sms * (s == 3 ? 90 : 82) / 100;
+            const int cap = occ == 2 ? sms * (s < 8 ? 184 : 173) / 100 : sms * (s == 4 ? 87 : s == 3 || s == 5 || s == 6 ? 90 : 82) / 100;
             if (s > 1 && tiles * s > cap) break;
             double us;
             if (s == 1 && bn >= 128 && can_persist && tiles > sms) {
@@ -1330,28 +1337,14 @@ bool jib_no_persist() {
     return off;
 }
 
-}  // namespace
-
-JIB_TL_DEFINE_SETTER(gemm)
-
-extern "C" JIB_EXPORT int jib_gemm_bf16(const jib_gemm_desc * d, void * stream_) {
-    cudaStream_t stream = (cudaStream_t) stream_;
-    if (d->T <= 0 || d->N <= 0 || d->K <= 0) return 0;
-    const bool dual = d->w2 != nullptr;
-    const bool grouped = d->seg != nullptr;
-    const int batch = d->batch > 0 ? d->batch : 1;
-    const bool src_mode = d->src_token != nullptr;
-    if (src_mode && (!grouped || d->src_rows <= 0 || d->src_rows > 256 || d->ar != nullptr)) return JIB_E_ARG;
-    const int rows_bound = src_mode ? d->src_rows : grouped ? (d->max_rows > 0 ? d->max_rows : d->T) : d->T;
-    if (narrow_ok(d, dual, batch)) return launch_narrow(d, dual, batch, stream);
-    int bn = d->bn;
-    if (bn == 0) {
-        bn = 16;
-        while (bn < rows_bound && bn < 256) bn *= 2;
-        if (dual && bn > 128) bn = 128;     // keeps three pipeline stages in shared memory
-    }
-    const int n_tiles = (d->N + BM - 1) / BM;
-    const int sms = d->sm_count > 0 ? d->sm_count : 148;
+// The kernel and, for planned products, the tiles that a descriptor leaves to the library.
+struct Form {
+    bool narrow, planned, vec_store;
+    TilePlan plan;
+};
+Form form_of(const jib_gemm_desc * d) {
+    const bool dual = d->w2 != nullptr, grouped = d->seg != nullptr;
+    const int batch = d->batch > 0 ? d->batch : 1, n_tiles = (d->N + BM - 1) / BM, sms = d->sm_count > 0 ? d->sm_count : 148;
     // 16-byte result stores: bf16 rows whose feature offsets keep 16-byte alignment (row pointers of the expert-parallel return
     // path are row starts of bf16 matrices with d % 8 == 0, hence aligned as well)
     bool vec_store = !d->out_f32 && d->N % 8 == 0 && d->ldo % 8 == 0 && d->out_batch_stride % 8 == 0 && ((uintptr_t) d->out & 15) == 0 &&
@@ -1363,16 +1356,49 @@ extern "C" JIB_EXPORT int jib_gemm_bf16(const jib_gemm_desc * d, void * stream_)
     // K, the larger the error of the tensor cores' sums (2048 x 2048 at 333 tokens: 4.7e-7 of the result in 4 splits, 2.1e-6 in one), which
     // a 16-bit result (1.7e-3) does not show.
     const bool planned = d->bn == 0 && d->splits <= 0 && !grouped && batch == 1 && d->ar == nullptr && d->ag_flags == nullptr &&
-                         !d->out_f32 && rows_bound > 32 && n_tiles <= 2 * sms;
-    TilePlan plan = {0, 0};
-    if (planned) {
-        plan = plan_tiles(d->N, d->K, rows_bound, dual, vec_store && !jib_no_persist(), sms);
-        bn = plan.bn;
+                         !d->out_f32 && d->T > 32 && n_tiles <= 2 * sms;
+    Form f = {narrow_ok(d, dual, batch), planned, vec_store, {0, 0}};
+    if (planned) f.plan = plan_tiles(d->N, d->K, d->T, dual, vec_store && !jib_no_persist(), sms);
+    return f;
+}
+
+}  // namespace
+
+JIB_TL_DEFINE_SETTER(gemm)
+
+extern "C" JIB_EXPORT int jib_gemm_form(const jib_gemm_desc * d, int * bn, int * splits) {
+    const Form f = form_of(d);
+    if (bn != nullptr) *bn = f.plan.bn;
+    if (splits != nullptr) *splits = f.plan.splits;
+    return f.narrow ? JIB_FORM_NARROW : f.planned ? JIB_FORM_PLANNED : JIB_FORM_RULES;
+}
+
+extern "C" JIB_EXPORT int jib_gemm_bf16(const jib_gemm_desc * d, void * stream_) {
+    cudaStream_t stream = (cudaStream_t) stream_;
+    if (d->T <= 0 || d->N <= 0 || d->K <= 0) return 0;
+    const bool dual = d->w2 != nullptr;
+    const bool grouped = d->seg != nullptr;
+    const int batch = d->batch > 0 ? d->batch : 1;
+    const bool src_mode = d->src_token != nullptr;
+    if (src_mode && (!grouped || d->src_rows <= 0 || d->src_rows > 256 || d->ar != nullptr)) return JIB_E_ARG;
+    const int rows_bound = src_mode ? d->src_rows : grouped ? (d->max_rows > 0 ? d->max_rows : d->T) : d->T;
+    const Form form = form_of(d);
+    if (form.narrow) return launch_narrow(d, dual, batch, stream);
+    int bn = d->bn;
+    if (bn == 0) {
+        bn = 16;
+        while (bn < rows_bound && bn < 256) bn *= 2;
+        if (dual && bn > 128) bn = 128;     // keeps three pipeline stages in shared memory
     }
+    const int n_tiles = (d->N + BM - 1) / BM;
+    const int sms = d->sm_count > 0 ? d->sm_count : 148;
+    const bool vec_store = form.vec_store, planned = form.planned;
+    const TilePlan plan = form.plan;
+    if (planned) bn = plan.bn;
     if (!planned && d->bn == 0 && bn == 256 && !grouped && d->ar == nullptr && !d->out_f32 && !jib_no_persist()) {
-        // Between one and two waves of 256-token tiles the second wave runs half empty and every CTA pays its prologue and
-        // epilogue in the open; the same product as 128-token tiles fills the persistent kernel's two to four rounds evenly
-        // with the epilogues hidden (2048 x 2048 x 2048: 25 us -> the persistent form).
+        // Products with a batch, explicit splits or a gather in front of them: between one and two waves of 256-token tiles the second wave
+        // runs half empty and every CTA pays its prologue and epilogue in the open; as 128-token tiles they fill the persistent kernel's two
+        // to four rounds evenly with the epilogues hidden.
         const long long t256 = (long long) n_tiles * ((rows_bound + 255) / 256) * batch;
         if (t256 < 2LL * sms && 4 * t256 >= 3LL * sms) bn = 128;
     }

@@ -77,6 +77,12 @@ typedef struct jib_gemm_desc {
 } jib_gemm_desc;
 
 JIB_EXPORT int jib_gemm_bf16(const jib_gemm_desc * d, void * stream);
+// Which form jib_gemm_bf16 takes for a descriptor, on the host and without a GPU: the kernel for up to 8 tokens, tiles chosen by the cost model
+// (token-tile width and splits in *bn, *splits), or the covering tile and the split rules.
+#define JIB_FORM_RULES 0
+#define JIB_FORM_PLANNED 1
+#define JIB_FORM_NARROW 2
+JIB_EXPORT int jib_gemm_form(const jib_gemm_desc * d, int * bn, int * splits);
 // The same product on CUDA cores (gemm_simt.cu): fp32 operands (f32 = 1, result fp32), or bf16 operands TMA cannot address.
 JIB_EXPORT int jib_gemm_simt(const jib_gemm_desc * d, int f32, void * stream);
 
