@@ -1107,7 +1107,7 @@ TilePlan plan_tiles(int N, int K, int T, bool dual, bool can_persist, int sms) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Products of up to 8 tokens with a matrix that one wave of CTAs holds in flight.  A tcgen05 tile of such a product is a chain of fixed
+// Products of up to 8 tokens with matrices of a few MB (see narrow_size).  A tcgen05 tile of such a product is a chain of fixed
 // costs (tensor memory, a ring of stages, the accumulator's way back, a cluster's sum: 4.5 to 7 us inside a decode graph for 1 to 8 MB
 // that take 0.2 to 1.3 us to read), so here a warp reads 16 rows straight into the fragments of m16n8k16 products, before the wait for the
 // previous kernel, and only the token rows (8 of them are the n of the product, whatever T is) and one barrier follow it.
@@ -1244,17 +1244,32 @@ int narrow_ks(int N, int K, int batch, int sms) {
     return ks;
 }
 
-// Where it is the faster of the two (us on a B200, weights from memory; N x K x heads, 1 / 8 tokens, tcgen05 tiles -> this): 128 x 512 x 16
-// 4.0 / 4.1 -> 2.5 / 2.7; 512 x 128 x 128 7.0 / 7.1 -> 5.2 / 5.8; 2048 x 512 4.0 / 4.1 -> 2.5 / 2.7; 4096 x 1024 4.2 / 4.5 -> 3.6 / 3.9; gated
-// pairs 512 x 512 8.3 / 7.6 -> 1.6 / 1.7, 1408 x 2048 5.4 / 5.8 -> 3.0 / 3.3, 5632 x 2048 15.1 / 16.5 -> 10.2 / 10.7.  Not where a row's run
-// is longer than the 256 elements a lane holds: rounds keep too little in flight (2112 x 5120 6.5 / 6.9 against 11.0 / 11.4), nor at that length
-// (2048 x 2048 4.3 / 4.5 against 4.4 / 4.9, and 3 us slower inside a decode graph); nor for matrices of several waves (128 x 512 x 128
-// 4.8 against 5.1 / 5.6, 32768 x 256 4.5 / 4.7 against 4.7 / 5.4, gated 8192 x 1536 10.0 / 11.2 against 11.7 / 12.1).
-// Whole passes: one conversation 74.8 -> 70.5 ms, four users of lugovik-lite 22.1 -> 21.4 ms.
-bool narrow_size(long long N, long long K, long long batch, bool dual) {
-    const long long mb = (N * K * batch * (dual ? 4 : 2)) >> 20;
-    if (dual) return K <= 2048 && mb < 47;
-    return K <= 128 ? mb <= 32 : K <= 1024 && mb < 12;
+// Whether the tcgen05 form of a product of one 16-token tile would add its splits up through memory, or in clusters that need a second wave
+// (see auto_splits and plan_tiles): 2 to 6 us either way.
+bool splits_badly(int N, int K, int batch, bool scratch, int sms) {
+    const long long tiles = (long long) ((N + BM - 1) / BM) * batch;
+    const int splits = scratch ? auto_splits(tiles, (K + BK - 1) / BK, 16, sms) : 1;
+    if (splits == 1) return false;
+    if (jib_no_cluster() || (tiles > 32 && splits > 4)) return true;
+    return tiles * (splits < 8 ? splits : 8) > 2LL * sms * 92 / 100;
+}
+
+// Where it is the faster of the two.  us on a B200, weights out of memory, between two small kernels of a graph, 8 tokens, tcgen05 tiles ->
+// this.  This form costs 2.0 us and 0.2 to 0.23 a MB.  One wave of tcgen05 tiles costs 2.8 us (K of 128), 3.1 (256: its ring takes the whole run),
+// 3.5 to 4.8 (longer), and a MB next to nothing up to 10 MB:
+//   K <= 256: up to 5 MB.  8192 x 256 (4 MB) 3.18 -> 2.88, 12288 x 256 (6) 3.08 -> 3.51; 512 x 128 x 32 heads (4) 2.92 -> 2.91
+//   K <= 1024: up to 9 MB.  8192 x 512 (8 MB) 4.12 -> 3.82, 10240 x 512 (10) 4.34 -> 4.76; 4096 x 1024 (8) 4.54 -> 3.89, 6144 x 1024 (12) 4.78 -> 5.08
+//   K <= 128 and more tiles than fit at a time: 40960 x 128 (320 tiles, 10 MB) 5.90 -> 4.26, 32768 x 128 (256 tiles, 8 MB) 3.07 -> 3.23;
+//   512 x 128 x 128 heads (512 tiles, 16 MB) 7.13 -> 5.59, and 49152 x 256 (384 tiles, 24 MB) 7.61 -> 8.62 is past it.
+// Longer rows: 2048 x 2048 4.18 -> 4.80.  Gated pairs have more of the fixed costs:
+//   up to 34 MB: 3072 x 2048 (24 MB) 6.62 -> 6.53, 7680 x 1024 (30) 8.12 -> 7.38, 4096 x 2048 (32) 8.37 -> 8.16, 10752 x 1024 (42) 9.90 -> 10.41
+//   where the tcgen05 tiles split badly up to 58 MB: 5632 x 2048 (44 MB) 15.97 -> 10.89, 7168 x 2048 (56) 16.34 -> 14.94, 7168 x 1536 (42) 14.20 ->
+//   11.96, 9216 x 1024 (36) 13.92 -> 8.78; next to them, with splits that fit: 7840 x 1536 (46) 9.96 -> 12.38, 8192 x 2048 (64) 12.99 -> 15.70.
+bool narrow_size(int N, int K, int batch, bool dual, bool scratch, int sms) {
+    const double mb = (double) N * K * batch * (dual ? 4 : 2) / (1 << 20);
+    if (dual) return K <= 2048 && (mb <= 34 || (mb <= 58 && splits_badly(N, K, batch, scratch, sms)));
+    if (K <= 128 && mb <= 16 && (long long) ((N + BM - 1) / BM) * batch > 2LL * sms) return true;
+    return K <= 1024 && mb <= (K <= 256 ? 5 : 9);
 }
 
 bool narrow_ok(const jib_gemm_desc * d, bool dual, int batch) {
@@ -1262,7 +1277,7 @@ bool narrow_ok(const jib_gemm_desc * d, bool dual, int batch) {
     return d->T <= NARROW_T && d->seg == nullptr && d->bn == 0 && d->splits <= 0 && d->ar == nullptr && d->ag_flags == nullptr && d->out_row_ptr == nullptr &&
            d->src_token == nullptr && d->K % 32 == 0 && d->x_row_stride % 8 == 0 && d->w_row_stride % 8 == 0 &&
            (batch == 1 || (d->x_batch_stride % 8 == 0 && d->w_batch_stride % 8 == 0)) && aligned(d->x) && aligned(d->w) && (!dual || aligned(d->w2)) &&
-           batch <= 65535 && narrow_size(d->N, d->K, batch, dual);
+           batch <= 65535 && narrow_size(d->N, d->K, batch, dual, d->scratch != nullptr, d->sm_count > 0 ? d->sm_count : 148);
 }
 
 int launch_narrow(const jib_gemm_desc * d, bool dual, int batch, cudaStream_t stream) {

@@ -26,6 +26,20 @@ def form(T, N, K, heads=1, gated=False, **more):
     return lib.jib_gemm_form(C.byref(d), bn, splits), bn.value, splits.value
 
 
+@pytest.mark.parametrize("N,K,heads,gated,narrow", [
+    (8192, 256, 1, False, True), (12288, 256, 1, False, False), (512, 128, 32, False, True), (128, 512, 16, False, True), (128, 512, 128, False, False),
+    (8192, 512, 1, False, True), (10240, 512, 1, False, False), (4096, 1024, 1, False, True), (6144, 1024, 1, False, False),
+    (40960, 128, 1, False, True), (32768, 128, 1, False, False), (512, 128, 128, False, True), (49152, 256, 1, False, False), (2048, 2048, 1, False, False),
+    (3072, 2048, 1, True, True), (4096, 2048, 1, True, True), (10752, 1024, 1, True, False), (7680, 1024, 1, True, True), (2048, 2080, 1, True, False),
+    (5632, 2048, 1, True, True), (7168, 2048, 1, True, True), (7168, 1536, 1, True, True), (9216, 1024, 1, True, True), (7840, 1536, 1, True, False),
+    (8192, 2048, 1, True, False)])
+def test_up_to_8_tokens(N, K, heads, gated, narrow):
+    for T in (1, 8):
+        assert form(T, N, K, heads, gated)[0] == (NARROW if narrow else RULES)
+    assert form(9, N, K, heads, gated)[0] == RULES
+    assert form(8, N, K, heads, gated, bn=16)[0] == form(8, N, K, heads, gated, splits=2)[0] == RULES
+
+
 def test_operands_that_16_byte_reads_do_not_fit():
     for more in ({"x": 4104}, {"w": 4104}, {"x_row_stride": 260}, {"w_row_stride": 260}, {"seg": 4096}):
         assert form(4, 1024, 256, **more)[0] == RULES, more
