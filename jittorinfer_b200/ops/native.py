@@ -42,7 +42,7 @@ EXPERT_LIST = os.environ.get("JIB_EXPERT_LIST", "1") == "1"
 TILE_LIST = os.environ.get("JIB_TILE_LIST", "1") == "1"
 TILE_LIST_MIN_PAIRS = 1024
 # Grouped launches of few rows per expert in tiles of 16 rows: for this many tokens; idle CTAs past which they walk a list.
-SMALL_TILES_MIN_T, SMALL_TILES_MAX_T, SMALL_TILES_MAX_IDLE = 24, 80, 20000
+SMALL_TILES_MIN_T, SMALL_TILES_MAX_T, SMALL_TILES_MAX_IDLE = 17, 80, 20000
 # The router launch of a decode batch also applies the RMSNorm of its input ("0": a separate norm launch before it).
 ROUTE_NORM = os.environ.get("JIB_ROUTE_NORM", "1") == "1"
 FUSED_ROUTE_MAX_T = 64
@@ -720,10 +720,13 @@ def moe_routed(x, ids, wts, wg, wu, wd, expert_base=0, n_expert=None, route=None
         # A dozen pairs an expert at most, nearly all experts hit: what counts is the stream of weights, and it runs best past tiles of 16
         # rows, two CTAs on an SM (64 tokens x 8 over 64 + 2 experts of 3 x 1408 x 2048: 208.7 us with every expert multiplying all 64 tokens,
         # 177.7 so, 177 at the rate of a copy; 32 tokens 186 -> 170, 77 tokens 190 -> 178; 160 + 2 experts of 3 x 1536 x 5120: 32 tokens 835 ->
-        # 776, 64 tokens 1088 -> 1011).  Below 24 tokens the rows in place are as fast, past 80 tiles of 128 rows.  The grid has a
-        # CTA for every tile that an expert could have; from some 20000 idle ones on (70 us at 25000) a list of the tiles is cheaper (6 us).
+        # 776, 64 tokens 1088 -> 1011).  Up to 16 tokens the rows in place are one tile of 16 as well and need no gather (16 tokens 134 us either
+        # way, 18 tokens 173 -> 157).  Past 80 tokens it depends on the shape: us at 88 tokens with tiles of 128 rows -> of 16: 64 + 2 experts
+        # 197 -> 186, 160 + 2 of 1536 x 5120 1154 -> 1168, 128 of 768 x 2048 200 -> 212, 32 + 1 of 1024 x 2048 84 -> 88; at 80: 195 -> 182,
+        # 1172 -> 1067, 199 -> 203, 81 -> 79 .. 85.  The grid has a CTA for every tile that an expert could have; from some 20000 idle ones on (70 us at
+        # 25000) a list of the tiles is cheaper (6 us).
         idle = E_local * ((T + 15) // 16 - 1) * ((wg.shape[1] + 127) // 128 + (wd.shape[1] + 127) // 128)
-        tl = moe_tile_list(seg, E_local, 16, T * k) if idle > SMALL_TILES_MAX_IDLE else None
+        tl = moe_tile_list(seg, E_local, 16, T * k) if TILE_LIST and idle > SMALL_TILES_MAX_IDLE else None
         h = gemm_grouped(gather_rows(x, src), seg, wg, wu, T, active, pdl_flags=pair[0], n_slots=slots, bn=16, tile_list=tl, gelu_scale=fn)
         return gemm_grouped(h, seg, wd, None, T, active, pdl_flags=pair[1], n_slots=slots, bn=16, tile_list=tl), dest
     if TILE_LIST and T * k >= TILE_LIST_MIN_PAIRS:

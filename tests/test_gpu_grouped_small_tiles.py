@@ -1,4 +1,4 @@
-"""Grouped expert products of 24 to 80 tokens in tiles of 16 rows: grid and list form, foreign experts and skewed routing against float64."""
+"""Grouped expert products of 17 to 80 tokens in tiles of 16 rows: grid and list form, foreign experts and skewed routing against float64."""
 import pytest
 import torch
 
@@ -15,8 +15,8 @@ def nat():
     native.check_status()
 
 
-# 23 and 81: the other paths; one row past tiles of 16; an expert with every token (five tiles) beside experts with none; the last sizes: the list
-@pytest.mark.parametrize("T,E,k,F,d,base", [(23, 20, 6, 192, 256, 0), (24, 20, 6, 192, 256, 0), (33, 66, 8, 136, 200, 0), (80, 66, 8, 192, 256, 0),
+# 16 and 81: the other paths; one row past tiles of 16; an expert with every token (five tiles) beside experts with none; the last sizes: the list
+@pytest.mark.parametrize("T,E,k,F,d,base", [(16, 20, 6, 192, 256, 0), (17, 20, 6, 192, 256, 0), (23, 20, 6, 192, 256, 0), (24, 20, 6, 192, 256, 0), (33, 66, 8, 136, 200, 0), (80, 66, 8, 192, 256, 0),
                                             (81, 66, 8, 192, 256, 0), (64, 24, 6, 192, 256, 40), (80, 160, 6, 1024, 3072, 0), (24, 256, 6, 128, 128, 0)])
 @pytest.mark.parametrize("gated", [True, False])
 def test_against_float64(nat, T, E, k, F, d, base, gated):
