@@ -162,13 +162,14 @@ __global__ void __launch_bounds__(GATE_NT) router_logits_kernel(const bf16 * __r
 // adjacent elements, warp g takes vector g of each (a lane: 4 tokens x 4 experts); the chunks of a span come in the order 0, 2, 1, 3 (vectors
 // g, g + 16, g + 8, g + 24: their sums are the first two levels), and the 8 warps' sums of a span meet in shared memory (the other three).
 // gridDim.z CTAs of a cluster take runs of spans; rank 0 adds their sums up in order.
-// Tiles of 16 tokens x 32 experts with three CTAs on an SM: 64 tokens x 64 experts are 8 tiles, and the chains of multiplications in front of every
-// addition need the warps (16 x 64, two CTAs: 16.5 against 10.7 us at 64 tokens, 44.0 against 41.3 at 2048).  Four stages: the same.  Router rows
-// of the first stages are requested before the wait for the previous kernel.
-// Router and gate on a B200, row kernel -> this (us): 64 experts x 2048: 17 tokens 10.4 -> 9.2, 64 17.1 -> 10.7, 333 35.0 -> 14.1, 2048 100 -> 41.3;
-// 160 x 5120: 17 tokens 22.1 -> 21.1, 64 56.8 -> 23.1, 2048 557 -> 193.  2-norm error against 64 bits as there: 0.99e-7 and 1.05e-7.  Sums in any
-// order that keeps packed pairs along d instead: 64 x 2048 9.9 us at 64 tokens, 32.8 at 2048, but errors of 1.04e-7 to 1.36e-7.
-constexpr int RT_T = 16, RT_E = 32, RT_J = RT_E / 8, RT_K = 64, RT_STAGES = 3, RT_NT = 256;
+// Tiles of 16 tokens x 32 experts: the chains of multiplications in front of every addition need registers, 16 x 64 spilled.  Two chunks share a
+// barrier, and a thread keeps a span's sums in registers until they meet.  Router rows of the first two are requested before the wait for the
+// previous kernel.
+// Router and gate on a B200, row kernel -> this (us): 64 experts x 2048: 17 tokens 10.4 -> 8.8, 64 17.1 -> 9.5,
+// 333 35.0 -> 14.4, 2048 100 -> 35.7; 160 x 5120: 17 tokens 22.1 -> 14.5, 64 56.8 -> 19.0, 2048 557 -> 186.
+// 2-norm error against 64 bits as there: 0.99e-7 (2048) and 1.05e-7 (5120).  Sums in an order of their own, packed in pairs along d: 9.9 us at 64
+// tokens, 32.8 at 2048, but errors of 1.04e-7 to 1.36e-7.
+constexpr int RT_T = 16, RT_E = 32, RT_J = RT_E / 8, RT_K = 64, RT_STAGES = 4, RT_NT = 256;
 constexpr int RT_SPAN = 256, RT_SPANS = 8, RT_TURN = RT_SPAN * RT_SPANS;     // elements of a span, spans, and what they cover together
 constexpr int RT_WROW = RT_K * 4 + 16, RT_GROW = RT_K * 2 + 16;            // padded rows: 8 experts (4 tokens) of a warp's read meet no bank twice
 constexpr int RT_STAGE = RT_E * RT_WROW + RT_T * RT_GROW;
@@ -193,7 +194,7 @@ struct RouterChunks {
 };
 
 template <bool ONE>      // one turn: d <= RT_TURN
-__global__ void __launch_bounds__(RT_NT, 3) router_tile_kernel(const bf16 * __restrict__ g, const float * __restrict__ w_router,
+__global__ void __launch_bounds__(RT_NT, 2) router_tile_kernel(const bf16 * __restrict__ g, const float * __restrict__ w_router,
                                                                float * __restrict__ logits, int T, int d, int E) {
     PDL_TRIGGER_TOP();
     extern __shared__ __align__(16) uint8_t rt_smem[];
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(RT_NT, 3) router_tile_kernel(const bf16 * __re
     const int s0 = n_spans * (int) blockIdx.z / S, s1 = n_spans * ((int) blockIdx.z + 1) / S;
     const uint32_t base = (uint32_t) __cvta_generic_to_shared(rt_smem);
     float * part = (float *) (rt_smem + RT_STAGES * RT_STAGE);             // [warp][token][expert ^ 8 (token mod 4)]
-    float * spans = part + (RT_NT / 32) * RT_OUT;                          // [span of this rank][token][expert]: ranks past 0
+    float * spans = part + (RT_NT / 32) * RT_OUT;                          // [span of this rank][token][expert]
     auto load_w = [&](int stage, int col) {      // rows past E and columns past d are zeros
         const uint32_t dst = base + stage * RT_STAGE;
 #pragma unroll
@@ -221,22 +222,25 @@ __global__ void __launch_bounds__(RT_NT, 3) router_tile_kernel(const bf16 * __re
             cp16_or_zero(dst + t * RT_GROW + k * 2, on ? g + (size_t) (t0 + t) * d + col + k : g, on);
         }
     };
+    // two chunks a stage pair: one barrier for both
     RouterChunks ahead = {d, s0, 0, 0};
-    int filled = 0;      // the stage that is filled next; used: the one that is read next
     {
         RouterChunks c = ahead;
-#pragma unroll
-        for (int s = 0; s < RT_STAGES - 1; ++s)
-            if (c.span < s1) { load_w(s, c.col()); c.next(); }
+        if (s0 < s1) {
+            load_w(0, c.col());
+            c.next();
+            load_w(1, c.col());
+        }
     }
     pdl_wait();      // inputs come from earlier kernels; nothing is written before this point
-#pragma unroll
-    for (int s = 0; s < RT_STAGES - 1; ++s) {
-        if (ahead.span < s1) { load_g(s, ahead.col()); ahead.next(); }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+    if (s0 < s1) {
+        load_g(0, ahead.col());
+        ahead.next();
+        load_g(1, ahead.col());
+        ahead.next();
     }
-    filled = RT_STAGES - 1;
-    int used = 0;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    int used = 0;      // the stage that is read next
     const int eg = lane & 7, tg = lane >> 3;      // experts eg + 8 j, tokens tg + 4 i
     float sum[RT_PER];
 #pragma unroll
@@ -256,18 +260,23 @@ __global__ void __launch_bounds__(RT_NT, 3) router_tile_kernel(const bf16 * __re
     };
     // acc += this warp's vector of the next chunk
     auto take = [&](float (&acc)[4][RT_J], int meet_span) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(RT_STAGES - 2) : "memory");
-        __syncthreads();      // the chunk is here for everybody, nobody reads the stage that is filled next, and all sums of meet_span are there
-        if (meet_span >= s0) meet(meet_span);
-        if (ahead.span < s1) {
-            load_w(filled, ahead.col());
-            load_g(filled, ahead.col());
-            ahead.next();
+        if (!(used & 1)) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();      // both chunks are here for everybody, nobody reads the stages that are filled next, and all sums of meet_span are there
+            if (ahead.span < s1) {
+                const int fill = used ^ 2;
+                load_w(fill, ahead.col());
+                load_g(fill, ahead.col());
+                ahead.next();
+                load_w(fill + 1, ahead.col());
+                load_g(fill + 1, ahead.col());
+                ahead.next();
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            }
+            if (meet_span >= s0) meet(meet_span);
         }
-        filled = filled + 1 == RT_STAGES ? 0 : filled + 1;
-        asm volatile("cp.async.commit_group;" ::: "memory");
         const uint8_t * st = rt_smem + used * RT_STAGE + warp * 32;
-        used = used + 1 == RT_STAGES ? 0 : used + 1;
+        used = (used + 1) & 3;
         float x[4][8];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -298,6 +307,7 @@ __global__ void __launch_bounds__(RT_NT, 3) router_tile_kernel(const bf16 * __re
     };
     for (int span = s0; span < s1; ++span) {
         const int turns = RouterChunks{d, span, 0, 0}.turns();
+        float u[4][RT_J];
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
             float v[4][RT_J];
@@ -323,23 +333,24 @@ __global__ void __launch_bounds__(RT_NT, 3) router_tile_kernel(const bf16 * __re
 #pragma unroll
                     for (int j = 0; j < RT_J; ++j) v[i][j] = __fadd_rn(v[i][j], y[i][j]);
             }
-            // the halves' sums in this thread's places; those of the span before were read two barriers ago at least
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < RT_J; ++j) {
-                    float & p = part[(warp * RT_T + tg + 4 * i) * RT_E + ((eg + 8 * j) ^ (8 * tg))];
-                    p = half == 0 ? v[i][j] : __fadd_rn(p, v[i][j]);
-                }
+                for (int j = 0; j < RT_J; ++j) u[i][j] = half == 0 ? v[i][j] : __fadd_rn(u[i][j], v[i][j]);
         }
+        // the sums of the span before were read a barrier ago
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < RT_J; ++j) part[(warp * RT_T + tg + 4 * i) * RT_E + ((eg + 8 * j) ^ (8 * tg))] = u[i][j];
     }
     __syncthreads();
     if (s1 > s0) meet(s1 - 1);
     if (S > 1) {      // each rank adds up a share of the results
         asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        const int share = RT_OUT / S;
-        if (tid < share) {
-            const int o = blockIdx.z * share + tid, t = t0 + o / RT_E, e = e0 + o % RT_E;
+        const int share = (RT_OUT + S - 1) / S, o = blockIdx.z * share + tid;
+        if (tid < share && o < RT_OUT) {
+            const int t = t0 + o / RT_E, e = e0 + o % RT_E;
             const uint32_t at = (uint32_t) __cvta_generic_to_shared(spans + o);
             float v[RT_SPANS], all = 0.f;
             int z = 0;
@@ -368,7 +379,7 @@ __global__ void __launch_bounds__(RT_NT, 3) router_tile_kernel(const bf16 * __re
 }
 
 // Which of the two: with few tokens the split over experts has more CTAs and shorter chains (64 x 2048, with the gate: 16 tokens 8.2 us there,
-// 17 tokens 10.4 there and 9.2 here).
+// 17 tokens 10.4 there and 8.8 here).
 constexpr int ROUTER_ROWS_MAX = 16;
 
 template <bool ONE>
@@ -377,9 +388,12 @@ int launch_router_tiles(const bf16 * g, const float * w_router, float * logits, 
     const int sms = jib::sm_count();
     if (sms <= 0 || !jib::ensure_dyn_smem(router_tile_kernel<ONE>, RT_SMEM, attr_done)) return JIB_E_LAUNCH;
     const dim3 tiles((E + RT_E - 1) / RT_E, (T + RT_T - 1) / RT_T);
-    // as many runs of spans (up to a portable cluster) as three CTAs per SM take at a time (twice as many: 777 x 64 x 2048 21.9 -> 26.7 us)
-    int S = 1;
-    while (S < 8 && (long long) tiles.x * tiles.y * 2 * S <= 3 * sms && 2 * S * RT_SPAN <= d) S *= 2;
+    // As many runs of spans (up to a portable cluster) as two CTAs per SM take at a time, some of which no cluster reaches (777 tokens x 64 x 2048: 196
+    // CTAs in pairs 21.8 us, 294 in threes 30.2); of the numbers with equally long runs the smallest.
+    const int n_spans = d < RT_TURN ? (d + RT_SPAN - 1) / RT_SPAN : RT_SPANS;
+    const long long room = 2LL * sms * 92 / 100 / ((long long) tiles.x * tiles.y);
+    int S = room < 1 ? 1 : room < n_spans ? (int) room : n_spans;
+    S = (n_spans + (n_spans + S - 1) / S - 1) / ((n_spans + S - 1) / S);
     if (jib::launch_pdl_cluster(router_tile_kernel<ONE>, dim3(tiles.x, tiles.y, S), dim3(RT_NT), RT_SMEM, stream, S, g, w_router, logits, T, d, E) !=
         cudaSuccess)
         return JIB_E_LAUNCH;
