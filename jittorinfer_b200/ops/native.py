@@ -216,9 +216,15 @@ def tensor_from_ptr(ptr: int, shape, dtype: torch.dtype, device) -> torch.Tensor
     return torch.as_tensor(_RawCudaBuffer(ptr, shape, typestr), device=device)
 
 
+# What torch.cuda.current_stream().cuda_stream gives, without the objects: a prompt of a few tokens is some 360 launches from Python.  Both names are
+# torch's own and private: a torch without them takes the objects.
+_raw_stream, _device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream() -> int:
-    # what torch.cuda.current_stream().cuda_stream gives, without the objects: a prompt of a few tokens is some 360 launches from Python
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    if _raw_stream is None or _device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_device())
 
 
 def _ck(rc: int, what: str):
