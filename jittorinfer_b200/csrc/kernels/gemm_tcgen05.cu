@@ -1583,7 +1583,7 @@ NoallocPlan noalloc_plan(int T, int N, int K, int splits, int sms) {
     while (p.bn < T && p.bn < 256) p.bn *= 2;
     p.n_tiles = (N + BM - 1) / BM;
     p.num_kb = (K + BK - 1) / BK;
-    if (splits <= 0) splits = auto_splits(p.n_tiles, p.num_kb, p.bn, sms);      // the rule jib_gemm_bf16 applies
+    if (splits <= 0) splits = auto_splits(p.n_tiles, p.num_kb, p.bn, sms);      // jib_gemm_bf16's rule for the covering tile
     if (splits > p.num_kb) splits = p.num_kb;
     p.kbps = (p.num_kb + splits - 1) / splits;
     p.splits = (p.num_kb + p.kbps - 1) / p.kbps;

@@ -14,7 +14,8 @@
 //
 // What it computes.  out[T][N] (bf16, row stride N) = x[T][K] (bf16, row stride K) times the
 // transpose of w[N][K] (bf16, row stride K), fp32 accumulation, with the K range cut into `splits`
-// parts (0 = let the library choose) exactly as jib_gemm_bf16 does.  T <= 256.
+// parts (0 = let the library choose).  T <= 256.  Tiles cover the tokens (a power of two of 16 to 256) and the partial sums meet in the array:
+// jib_gemm_bf16 with that tile width and the same explicit count gives the same products, added up in the same parts.
 //
 // Limits and errors.  The partial sums need
 //     ceil(N/128) * splits * max(16, pow2ceil(T)) * 128 * 4 bytes  <=  JIB_NOALLOC_SCRATCH_BYTES
@@ -22,7 +23,8 @@
 // JIB_E_NOALLOC_TOO_LARGE and launches nothing.  Other failures the host can see (bad arguments,
 // alignment, a refused launch) return the JIB_E_* codes of jib_kernels.h.  Pointers must be 16-byte
 // aligned and K a multiple of 8.  With splits = 0 the count follows the SM count of the current
-// device (queried once per device), by the same rule as jib_gemm_bf16.
+// device (queried once per device), by the rule that jib_gemm_bf16 has for the covering tile.  That call itself may choose
+// otherwise when it is free to: a kernel of its own up to 8 tokens, tiles and splits by a cost model past 32 (jib_gemm_form).
 //
 // Faults found on the device.  The kernel's waits are bounded and its scratch indices checked; when
 // a wait runs out or an index is out of range it records a code in four status words inside the
