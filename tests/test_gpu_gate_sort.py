@@ -70,7 +70,7 @@ def test_one_launch(nat, T, E, k, n_shared, n_group, topk_group, top2, sigmoid, 
 
 
 def test_no_numbers_and_infinities(nat):
-    """Scores that are all NaN pick expert 0; fewer numbers than choices re-pick the lowest masked one."""
+    """Scores that are all NaN pick expert 0; logits of minus infinity are probabilities of 0, taken in order of their ids."""
     E, k = 40, 4
     logits = torch.zeros(3, E, device=DEV)
     logits[0] = float("nan")
@@ -84,6 +84,33 @@ def test_no_numbers_and_infinities(nat):
     assert ids[0].tolist() == [0, 0, 0, 0]
     assert ids[1].tolist() == [7, 0, 1, 2] and wts[1].tolist() == [1.0, 0.0, 0.0, 0.0]
     assert ids[2].tolist() == [5, 33, 0, 1]
+
+
+@pytest.mark.parametrize("E,n_group,k", [(32, 8, 6), (64, 16, 8), (256, 32, 31), (40, 20, 4)])
+@pytest.mark.parametrize("top2", [False, True])
+def test_fewer_eligible_experts_than_choices(nat, E, n_group, k, top2):
+    """One group of E / n_group experts is left; the choices past them re-pick the lowest masked id, 0, with its own weight."""
+    T, gs = 5, E // n_group
+    logits = torch.randn(T, E, generator=torch.Generator().manual_seed(E)) * 2
+    p = torch.softmax(logits.double(), -1)
+    want = torch.zeros(T, k, dtype=torch.long)
+    for t in range(T):
+        score = p[t].view(n_group, gs)
+        best = int((score.topk(2, -1).values.sum(-1) if top2 else score.max(-1).values).argmax())
+        mine = sorted(range(best * gs, best * gs + gs), key=lambda e: (-float(p[t, e]), e))
+        want[t, :gs] = torch.tensor(mine)
+    dev = logits.to(DEV)
+    ids, wts = torch.empty(T, k, dtype=torch.int32, device=DEV), torch.empty(T, k, device=DEV)
+    nat._ck(nat.load().jib_moe_gate(None, None, None, None, dev.data_ptr(), ids.data_ptr(), wts.data_ptr(), T, 8, E, k, n_group, 1, 1.0, 0, 0, 0, int(top2), 0,
+                                    nat._stream()), "moe_gate")
+    assert torch.equal(ids.long().cpu(), want)
+    assert bool(((wts.double().cpu() - p.gather(1, want)).abs() <= 1e-6 * p.gather(1, want)).all())
+    both, rows = torch.empty_like(ids), torch.empty_like(wts)
+    seg, src, dest = (torch.empty(n, dtype=torch.int32, device=DEV) for n in (2 * E + 1, T * k, T * k))
+    nat._ck(nat.load().jib_moe_gate_sort(None, None, None, None, dev.data_ptr(), both.data_ptr(), rows.data_ptr(), T, 8, E, k, n_group, 1, 1.0, 0, 0, 0,
+                                         int(top2), 0, 0, E, seg.data_ptr(), src.data_ptr(), dest.data_ptr(), None, nat._stream()), "moe_gate_sort")
+    assert torch.equal(both, ids) and torch.equal(rows, wts)
+    check_sort(ids, 0, E, seg[:E + 1], src, dest.view(T, k))
 
 
 @pytest.mark.parametrize("T,k,E,base", [(77, 8, 66, 0), (128, 8, 66, 0), (129, 31, 256, 100), (511, 8, 256, 0), (1, 1, 1, 0)])

@@ -4,6 +4,9 @@ import types
 import pytest
 import torch
 
+from jittorinfer_b200.ops import reference as ref
+from jittorinfer_b200.ops.specs import Gqa
+
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
@@ -57,3 +60,43 @@ def test_decode(nat, H, G, window, lens):
         # probabilities and the result are rounded to bf16 (half of 2^-8 each), sums and exponentials to fp32
         lim = 2.0 ** -8 * torch.einsum("hn,nhd->hd", p, v.abs()) + 2.0 ** -8 * want.abs() + 1e-5
         assert bool(((got - want).abs() <= lim).all()), float(((got - want).abs() / lim).max())
+
+
+# the loop's branches, each in batches with a dry round (3 sequences) and without one (300)
+@pytest.mark.parametrize("n", [3, 300])
+@pytest.mark.parametrize("option", [dict(chunk=96), dict(softcap=2.5), dict(sink=True), dict(sink=True, softcap=2.5, window=70), dict(gate=1), dict(gate=2, chunk=64),
+                                    dict(window=70, pool=16), dict(window=33, pool=7, sink=True, gate=2)])
+def test_options(nat, option, n):
+    H, G, D = 8, 2, 128
+    option = dict(option)
+    gate = option.pop("gate", 0)
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    m = Gqa(H, G, D, D, D, 0.09, gate_each=gate == 2, **option)
+    if m.sink:
+        m.sink_w = torch.randn(H, generator=gen, device=DEV)
+    lens = [(200, 1, 97)[i] if i < 3 else 5 + i % 190 for i in range(n)]
+    nb = [(s + 63) // 64 for s in lens]
+    bt = torch.zeros(n, 6, dtype=torch.int32)
+    at = 1
+    for i, k in enumerate(nb):
+        bt[i, :k] = torch.arange(at, at + k)
+        at += k
+    bt = bt.to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)      # noqa: E731
+    rows = lambda k: torch.randn(k, m.kv_row, generator=gen, device=DEV).bfloat16()      # noqa: E731
+    cache, pool = rows(at * 64), rows(at * m.pool_rows(64)) if m.pool else None
+    q = torch.randn(n, H, D, generator=gen, device=DEV).bfloat16()
+    g = torch.randn(n, H * (D if gate == 2 else 1), generator=gen, device=DEV).bfloat16() if gate else None
+    out, want, size = (torch.zeros(n, H * D, dtype=t, device=DEV) for t in (torch.bfloat16, torch.float32, torch.float32))
+    args = (bt, i32(lens), i32(list(range(n + 1))), 64, 1, None)
+    for _ in range(2):
+        nat.gqa_attention(m, q, cache, g, *args, out, pool)
+    ref.gqa_attention(m, q, cache, g, *args, want, pool)
+    # |v| in the values' place bounds the sums that the rounded probabilities go into
+    both = [t.float() for t in (cache, pool) if t is not None]
+    for t in both:
+        t[:, G * D:] = t[:, G * D:].abs()
+    ref.gqa_attention(m, q, both[0], g, *args, size, both[1] if m.pool else None)
+    # probabilities and the result are rounded to bf16 (half of 2^-8 each); gates and the softcap's tanh by fast functions (2^-20 of a score)
+    lim = 2.0 ** -8 * size + 2.0 ** -8 * want.abs() + 1e-4
+    assert bool(((out.float() - want).abs() <= lim).all()), float(((out.float() - want).abs() / lim).max())
