@@ -8,15 +8,6 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.fixture(scope="module")
-def nat():
-    from jittorinfer_b200.ops import native
-    native.load()
-    yield native
-    torch.cuda.synchronize()
-    native.check_status()
-
-
 def check_sort(ids, base, E_local, seg, src, dest):
     T, k = ids.shape
     flat = ids.flatten().long().cpu() - base

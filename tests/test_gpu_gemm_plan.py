@@ -6,15 +6,6 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.fixture(scope="module")
-def nat():
-    from jittorinfer_b200.ops import native
-    native.load()
-    yield native
-    torch.cuda.synchronize()
-    native.check_status()
-
-
 def bounded(y, ref, x, w, K):
     """Rounding of the result (bf16: half of 2^-8; twice that, for the activation's own rounding) plus fp32 sums of K products."""
     eps = 2.0 ** -8 if y.dtype == torch.bfloat16 else 2.0 ** -22

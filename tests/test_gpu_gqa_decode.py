@@ -11,15 +11,6 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.fixture(scope="module")
-def nat():
-    from jittorinfer_b200.ops import native
-    native.load()
-    yield native
-    torch.cuda.synchronize()
-    native.check_status()
-
-
 def mixer(H, G, window=0):
     return types.SimpleNamespace(heads=H, kv_heads=G, dim=128, vdim=128, rot=128, window=window, chunk=0, sink=False, scale=0.09, softcap=0.0, eps=1e-6,
                                  out_scale=1.0, sink_w=None, neighbours=False, unit=False, gate_each=False, pool=0)

@@ -6,15 +6,6 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.fixture(scope="module")
-def nat():
-    from jittorinfer_b200.ops import native
-    native.load()
-    yield native
-    torch.cuda.synchronize()
-    native.check_status()
-
-
 # 16 and 81: the other paths; one row past tiles of 16; an expert with every token (five tiles) beside experts with none; the last sizes: the list
 @pytest.mark.parametrize("T,E,k,F,d,base", [(16, 20, 6, 192, 256, 0), (17, 20, 6, 192, 256, 0), (23, 20, 6, 192, 256, 0), (24, 20, 6, 192, 256, 0), (33, 66, 8, 136, 200, 0), (80, 66, 8, 192, 256, 0),
                                             (81, 66, 8, 192, 256, 0), (64, 24, 6, 192, 256, 40), (80, 160, 6, 1024, 3072, 0), (24, 256, 6, 128, 128, 0)])

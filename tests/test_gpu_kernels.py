@@ -10,15 +10,6 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.fixture(scope="module")
-def nat():
-    from jittorinfer_b200.ops import native
-    native.load()
-    yield native
-    torch.cuda.synchronize()
-    native.check_status()
-
-
 def rnd(*shape, scale=1.0, dtype=torch.bfloat16, seed=None):
     g = torch.Generator(device="cpu")
     g.manual_seed(hash(shape) % (2 ** 31) if seed is None else seed)
@@ -303,6 +294,7 @@ def test_fused_route_matches_the_separate_kernels(nat, T, d, E, k, n_group, topk
             nat.FUSED_ROUTE = True
             res = nat.moe_gate(y, w_router, None, k, n_group, topk_group, 1.0, False, False, n_shared, False, (base, E_local), pre)
             ids1, wts1 = res[0], res[1]
+            assert len(nat._route_stash) == 1                 # the one launch ran
             seg1, src1, dest1 = nat.moe_permute(ids1, base, E_local)
             torch.cuda.synchronize()
             assert not nat._route_stash                       # the sort came from the fused launch

@@ -8,15 +8,6 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.fixture(scope="module")
-def nat():
-    from jittorinfer_b200.ops import native
-    native.load()
-    yield native
-    torch.cuda.synchronize()
-    native.check_status()
-
-
 def rnd(*shape, seed, scale=1.0):
     g = torch.Generator(device=DEV).manual_seed(seed)
     return (torch.randn(*shape, generator=g, device=DEV) * scale).bfloat16()

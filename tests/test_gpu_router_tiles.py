@@ -6,15 +6,6 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.fixture(scope="module")
-def nat():
-    from jittorinfer_b200.ops import native
-    native.load()
-    yield native
-    torch.cuda.synchronize()
-    native.check_status()
-
-
 # 16: the other kernel; one past a tile of 16 tokens, several tiles, more tiles than CTA slots; experts below, at and past a tile of 64;
 # widths of less than one chunk of 64, a ragged one, one run of many chunks
 @pytest.mark.parametrize("T", [1, 16, 17, 33, 77, 2049])
